@@ -288,7 +288,8 @@ __global__ void __launch_bounds__(128) row_moments_kernel(ColPass a, MomentSpec 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Direct-DFT fallback for lengths the four-step kernels do not cover (O(n^2) per line).
+// Direct-DFT fallback (O(n^2) per line) for lengths neither the four-step kernels nor the
+// any-length passes cover: 1, and above 3128.
 // ------------------------------------------------------------------------------------------------
 template <bool INV> __device__ __forceinline__ float2 unit_root(int64_t m, int n) {
   float s, c;
@@ -444,6 +445,8 @@ int launch_row_pass(const RowPass &a, int nwin, cudaStream_t s) {
       HF_DISPATCH_N1(a.N, return (launch_row_fast<N1, false>(a, nwin, s)))
     }
   }
+  if (fft_any_length(a.N))
+    return launch_row_any(a, nwin, s);
   const int64_t total = (int64_t)a.nplanes * a.H * a.N;
   if (a.inverse)
     row_dft_generic_kernel<true><<<dim3(grid_for(total, 256), nwin), 256, 0, s>>>(a);
@@ -470,6 +473,8 @@ int launch_col_pass(const ColPass &a, int mode, const MomentSpec *mom, int nwin,
   }
   if (mode != COL_COMPLEX && mode != COL_MAGNITUDE)
     return fail(HF_ERR_UNSUPPORTED, "fused column mode needs a four-step length");
+  if (fft_any_length(a.H))
+    return launch_col_any(a, mode == COL_MAGNITUDE, nwin, s);
   const int64_t total = (int64_t)a.nplanes * a.H * a.W;
   if (a.inverse)
     col_dft_generic_kernel<true><<<dim3(grid_for(total, 256), nwin), 256, 0, s>>>(a, mode == COL_MAGNITUDE);

@@ -61,6 +61,10 @@ enum ColMode { COL_COMPLEX = 0, COL_MAGNITUDE = 1, COL_MOMENTS = 2, COL_TF_SANDW
 
 // Whether the fused four-step kernels cover transform length n (n = 32 * N1).
 bool fft_fast_length(int n);
+// Whether the any-length passes (k_fft_any.cu) cover transform length n.
+bool fft_any_length(int n);
+int  launch_row_any(const RowPass &a, int nwin, cudaStream_t s);
+int  launch_col_any(const ColPass &a, int magnitude, int nwin, cudaStream_t s);
 
 int launch_row_pass(const RowPass &a, int nwin, cudaStream_t s);
 int launch_col_pass(const ColPass &a, int mode, const MomentSpec *mom, int nwin, cudaStream_t s);

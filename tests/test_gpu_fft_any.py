@@ -1,0 +1,86 @@
+"""Any-length row and column passes (k_fft_any.cu) against the float64 oracle: edges of the radix
+sets (primes with a register butterfly, larger primes through the dense stage, composite radices),
+lengths around the shared-memory limit, partial row groups and strips, and every form the passes
+take (real and strided input, strided output, output lens, inverse, placement in a padded plane)."""
+import math
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+LAM, DX = 852e-9, 12e-6
+
+
+def _tol(*sides):
+    # one rounding of 2^-24 per stage level, sqrt(p) of them in a dense stage of prime p; the bound
+    # of the four-step passes, 2e-6 log2(HW), covers both up to the longest length
+    return 2e-6 * math.log2(math.prod(sides))
+
+
+@pytest.mark.parametrize("H,W", [(2, 3), (5, 17), (19, 23), (37, 48), (90, 98), (109, 218), (480, 640), (600, 800),
+                                 (601, 17), (9, 601), (387, 218), (1013, 12), (7, 2048), (2048, 5), (3, 3128),
+                                 (3128, 3), (4, 3121), (2, 3200)])
+@pytest.mark.parametrize("mode", ["complex", "magnitude", "phase"])
+def test_fresnel_any_sides(cuda, H, W, mode):
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(H * 10007 + W)
+    B = 3
+    x = (rng.standard_normal((B, H, W)) + 1j * rng.standard_normal((B, H, W))).astype(np.complex64)
+    mag, skip = mode == "magnitude", mode != "phase"
+    plan = pl.FresnelPlan(B, H, W, hf.HF_CF32, LAM, DX, 0.3, output_magnitude=mag, skip_phase_shift=skip)
+    got = plan(torch.from_numpy(x).to(cuda)).cpu().numpy()
+    exp = O.fresnel(x, LAM, DX, DX, 0.3, output_magnitude=mag, skip_phase_shift=skip)
+    assert O.rel_l2(got, exp) < _tol(H, W)
+
+
+def test_fresnel_any_real_strided_in_and_out(cuda):
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(1)
+    big = rng.standard_normal((2, 75, 2 * 106)).astype(np.float32)
+    dev = torch.from_numpy(big).to(cuda)[:, :, ::2]
+    for mag, dt in ((True, torch.float32), (False, torch.complex64)):
+        plan = pl.FresnelPlan(2, 75, 106, hf.HF_F32, LAM, DX, 0.2, output_magnitude=mag)
+        wide = torch.zeros((2, 75, 3 * 106), dtype=dt, device=cuda)
+        plan(dev, out=wide[:, :, ::3])
+        exp = O.fresnel(big[:, :, ::2], LAM, DX, DX, 0.2, output_magnitude=mag)
+        w = wide.cpu().numpy()
+        assert O.rel_l2(w[:, :, ::3], exp) < _tol(75, 106)
+        assert not w[:, :, 1::3].any() and not w[:, :, 2::3].any()
+
+
+@pytest.mark.parametrize("B,H,W,pad,real", [(2, 50, 70, None, False), (1, 33, 57, (61, 41), True),
+                                            (2, 101, 37, (59, 151), False), (1, 600, 480, None, True)])
+def test_angular_spectrum_any_sides(cuda, B, H, W, pad, real):
+    """Forward and inverse transforms of both axes, with placement in a padded plane."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(2)
+    x = rng.standard_normal((B, H, W)).astype(np.float32)
+    if not real:
+        x = (x + 1j * rng.standard_normal((B, H, W))).astype(np.complex64)
+    padding = {"width": pad[0], "height": pad[1]} if pad else None
+    plan = pl.AngularSpectrumPlan(B, H, W, hf.HF_F32 if real else hf.HF_CF32, LAM, DX, 0.3, padding, None)
+    got = plan(torch.from_numpy(x).to(cuda)).cpu().numpy()
+    exp = O.angular_spectrum(x, LAM, DX, DX, 0.3, None, padding)
+    assert O.rel_l2(got, exp) < 5e-5
+
+
+def test_overflowing_squares_keep_their_magnitude(cuda):
+    """|v| of values whose squares leave the float32 range, as hypot gives it."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    for scale in (1e25, 1e-25):
+        x = np.zeros((1, 5, 7), np.complex64)
+        x[0, 2, 3] = scale
+        plan = pl.FresnelPlan(1, 5, 7, hf.HF_CF32, LAM, DX, 0.3, output_magnitude=True)
+        got = plan(torch.from_numpy(x).to(cuda)).cpu().numpy()
+        np.testing.assert_allclose(got, np.full((1, 5, 7), scale), rtol=1e-5)
