@@ -57,7 +57,8 @@ enum { HF_PROP_NONE = 0, HF_PROP_FRESNEL = 1, HF_PROP_ANGULAR_SPECTRUM = 2 };
 /* Moment selection bits (holovibes MomentType M0/M1/M2, graph_builder.cc:604-631) */
 enum { HF_M0 = 1, HF_M1 = 2, HF_M2 = 4 };
 
-/* Numeric form of the pipeline: all-FP32 ("plain") or tensor-core ("chosen") */
+/* Numeric form of the pipeline: FP32 ("plain"; the Gram matrix of 8/12-bit frames in exact integers)
+ * or tensor-core ("chosen") */
 enum { HF_FORM_PLAIN = 0, HF_FORM_CHOSEN = 1 };
 
 /* ---- library ------------------------------------------------------------------------------ */
