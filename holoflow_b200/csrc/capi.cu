@@ -83,16 +83,12 @@ int hf_temporal_dft(const void *in, int in_dtype, int64_t batch, int T, int64_t 
                      frame_bytes_of(in_dtype, P)};
   a.T           = T;
   a.P           = P;
-  a.H           = 1;
-  a.W           = (int)P;
   a.nz          = z1 - z0;
   a.wmat        = nullptr;
   a.z0          = z0;
   a.wmat_stride = 0;
   a.lens        = nullptr;
   a.out         = reinterpret_cast<float2 *>(out);
-  a.OH          = 1;
-  a.OW          = (int)P;
   a.out_plane   = P;
   a.out_win     = (int64_t)(z1 - z0) * P;
   a.scale       = norm_scale(norm, T);

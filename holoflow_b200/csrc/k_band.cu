@@ -1,6 +1,5 @@
 // Temporal band DFT: per pixel S_k = scale * sum_t x_t W[t][k] for k < nz, written as complex
-// planes [nz][OH][OW] (optionally multiplied by a per-pixel lens and placed at an offset inside
-// a larger zero-padded plane).
+// planes [nz][P] (optionally multiplied by a per-pixel lens).
 //
 // W is the T x nz complex matrix a window's SVD clutter filter and its band DFT reduce to,
 // W = (I - V V^T) D[:, z0:z1]  (D the unnormalised DFT, V the removed eigenvectors), so this one
@@ -8,8 +7,19 @@
 // fft.cu:234-252, graph_builder.cc:264-267) and for the filter, and Fresnel's lens multiply
 // (the load callback of fresnel_diffraction.cu:262-303) is fused into its store.
 //
-// Plain form: FP32 CUDA-core FMAs.  A CTA stages the packed samples of a 1024-pixel tile for all
-// T frames in shared memory once, then each thread accumulates 7 bins x 8 pixels in registers.
+// Plain form: FP32 CUDA-core FMAs, and their rate is the bound: T nz complex-by-real products per
+// pixel, 60 GFLOP for 8 windows of 64 x 1024^2 at nz = 28 (0.83 ms at 72 TFLOP/s).
+//  - A thread holds NB bins x 4 pixels of complex sums; (re, im) is one packed fp32x2 FMA, so a
+//    frame costs 4 NB packed FMAs against NB / 2 broadcast loads of W, two loads of samples and
+//    about 20 instructions of unpacking.  7 bins x 8 pixels with scalar FMAs and integer-to-float
+//    conversions took 2.82 ms for those 8 windows.
+//  - Integer samples are taken as x - shift (exact; no conversion instruction), and shift sum_t W is
+//    added at the end: the running sums stay small, so they round less than sums of raw samples.
+//  - 128 threads per CTA, three CTAs per SM (about 170 registers each): 128 / KG lanes x 4 pixels by
+//    KG bin groups.  The CTAs are persistent over the pixel tiles of a window, so W is staged once,
+//    and the next tile's samples stream in by cp.async while this one is summed.
+#include <algorithm>
+
 #include "frames.cuh"
 #include "k_band.cuh"
 
@@ -17,46 +27,41 @@ namespace hf {
 
 namespace {
 
-constexpr int kBandNB  = 7;   // bins per thread
-constexpr int kBandPX  = 8;   // pixels per thread
-constexpr int kBandHalf = 2;  // bin chunks processed side by side by the two halves of a CTA
+constexpr int kBandPX  = 4;   // pixels per thread
+constexpr int kBandThr = 128;
 
 template <int FMT> struct FmtBytes;
-template <> struct FmtBytes<HF_MONO12P> { static constexpr int num = 3, den = 2; };
-template <> struct FmtBytes<HF_U16> { static constexpr int num = 2, den = 1; };
-template <> struct FmtBytes<HF_U8> { static constexpr int num = 1, den = 1; };
-template <> struct FmtBytes<HF_F32> { static constexpr int num = 4, den = 1; };
+template <> struct FmtBytes<HF_MONO12P> { static constexpr int num = 3, den = 2; static constexpr float shift = 2048.f; };
+template <> struct FmtBytes<HF_U16> { static constexpr int num = 2, den = 1; static constexpr float shift = 2048.f; };
+template <> struct FmtBytes<HF_U8> { static constexpr int num = 1, den = 1; static constexpr float shift = 128.f; };
+template <> struct FmtBytes<HF_F32> { static constexpr int num = 4, den = 1; static constexpr float shift = 0.f; };
 
-// 8 consecutive samples of one frame from the staged tile (words, 4-byte aligned)
-template <int FMT>
-__device__ __forceinline__ void load8(const uint32_t *row, int g, float (&x)[kBandPX]) {
-  if constexpr (FMT == HF_MONO12P) {
-    uint32_t p[8];
-    unpack8(row[3 * g], row[3 * g + 1], row[3 * g + 2], p);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      x[i] = (float)p[i];
+// Integer sample v < 2^23 as the float v - shift, exactly: (2^23 + v) - (2^23 + shift).
+template <int FMT> __device__ __forceinline__ float centred(uint32_t v) {
+  return __uint_as_float(0x4B000000u | v) - (8388608.f + FmtBytes<FMT>::shift);
+}
+
+// Samples 4 g .. 4 g + 3 of a staged row, minus the shift.
+template <int FMT> __device__ __forceinline__ void load4(const uint8_t *row, int g, float (&x)[kBandPX]) {
+  if constexpr (FMT == HF_MONO12P) { // 48 bits from bit 0 (even g) or 16 (odd g) of two words
+    const uint32_t *w  = reinterpret_cast<const uint32_t *>(row) + 3 * (g >> 1) + (g & 1);
+    const uint32_t  a = w[0], b = w[1], sh = (g & 1) * 16;
+    const uint32_t  lo = __funnelshift_r(a, b, sh), hi = b >> sh;
+    x[0] = centred<FMT>(lo & 0xFFFu);
+    x[1] = centred<FMT>((lo >> 12) & 0xFFFu);
+    x[2] = centred<FMT>(__funnelshift_r(lo, hi, 24) & 0xFFFu);
+    x[3] = centred<FMT>((hi >> 4) & 0xFFFu);
   } else if constexpr (FMT == HF_U16) {
-    const uint4 v = reinterpret_cast<const uint4 *>(row)[g];
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      x[2 * i]     = (float)(w[i] & 0xFFFFu);
-      x[2 * i + 1] = (float)(w[i] >> 16);
-    }
-  } else if constexpr (FMT == HF_U8) {
     const uint2 v = reinterpret_cast<const uint2 *>(row)[g];
-    const uint32_t w[2] = {v.x, v.y};
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        x[4 * i + j] = (float)((w[i] >> (8 * j)) & 0xFFu);
+    x[0] = centred<FMT>(v.x & 0xFFFFu), x[1] = centred<FMT>(v.x >> 16);
+    x[2] = centred<FMT>(v.y & 0xFFFFu), x[3] = centred<FMT>(v.y >> 16);
+  } else if constexpr (FMT == HF_U8) {
+    const uint32_t v = reinterpret_cast<const uint32_t *>(row)[g];
+    x[0] = centred<FMT>(v & 0xFFu), x[1] = centred<FMT>((v >> 8) & 0xFFu);
+    x[2] = centred<FMT>((v >> 16) & 0xFFu), x[3] = centred<FMT>(v >> 24);
   } else { // F32
-    const float4 a = reinterpret_cast<const float4 *>(row)[2 * g];
-    const float4 b = reinterpret_cast<const float4 *>(row)[2 * g + 1];
-    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
-    x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    const float4 v = reinterpret_cast<const float4 *>(row)[g];
+    x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
   }
 }
 
@@ -70,95 +75,139 @@ __device__ __forceinline__ float2 wmat_entry(const BandArgs &a, int w, int t, in
   return make_float2(c, s);
 }
 
-template <int FMT>
-__global__ void __launch_bounds__(256) band_dft_tiled_kernel(BandArgs a, int tile_px) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  constexpr int num = FmtBytes<FMT>::num, den = FmtBytes<FMT>::den;
-  const int     w         = blockIdx.y;
-  const int64_t tile0     = (int64_t)blockIdx.x * tile_px;
-  const int     row_bytes = tile_px * num / den;
-  const int     row_words = row_bytes / 4;
-  const int     groups    = tile_px / kBandPX; // threads per bin chunk
-  const int     nzpad     = ((a.nz + kBandNB * kBandHalf - 1) / (kBandNB * kBandHalf)) * kBandNB * kBandHalf;
-
-  uint32_t *tile  = reinterpret_cast<uint32_t *>(smem);
-  float2   *w_sh  = reinterpret_cast<float2 *>(smem + (size_t)a.T * row_bytes);
-  float2   *lens  = w_sh + (size_t)a.T * nzpad;
-
-  const int tid = threadIdx.x;
-  // stage the packed tile of every frame (4-byte words, coalesced per frame)
-  const int64_t tile_byte0 = tile0 * num / den;
-  const int64_t valid_px   = min((int64_t)tile_px, a.P - tile0);
-  const int     valid_words = (int)(valid_px * num / den + 3) / 4;
-  // asynchronous 4-byte copies: every frame's words are in flight at once instead of one
-  // load-then-store at a time (the tail beyond the image is zero-filled, src-size 0)
-  for (int t = 0; t < a.T; ++t) {
-    const uint32_t *src = reinterpret_cast<const uint32_t *>(a.ring.frame(w, t) + tile_byte0);
-    for (int i = tid; i < row_words; i += blockDim.x) {
-      const bool     ok  = i < valid_words;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(tile + t * row_words + i);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(ok ? src + i : src),
-                   "r"(ok ? 4 : 0)
-                   : "memory");
+// Copies `bytes` bytes of a row into shared memory (16-byte aligned), zero beyond `valid`.  `unit` is
+// the common alignment of every row of the tile: 16 and 4 go by cp.async, less byte by byte.
+__device__ __forceinline__ void stage_tile(uint8_t *dst, const uint8_t *base, const int64_t *foff, int T, int bytes,
+                                           int valid, int unit) {
+  if (unit >= 4) {
+    const int per = bytes / unit;
+    for (int i = threadIdx.x; i < T * per; i += kBandThr) {
+      const int      t = i / per, o = (i - t * per) * unit, n = max(0, min(unit, valid - o));
+      const uint8_t *src = base + foff[t] + (n > 0 ? o : 0);
+      const uint32_t d   = (uint32_t)__cvta_generic_to_shared(dst + t * bytes + o);
+      if (unit == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    }
+  } else {
+    constexpr int U = 8; // loads in flight per thread
+    for (int i0 = threadIdx.x; i0 < T * bytes; i0 += U * kBandThr) {
+      uint8_t v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * kBandThr, t = i / bytes, o = i - t * bytes;
+        v[u]        = i < T * bytes && o < valid ? __ldg(base + foff[t] + o) : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * kBandThr < T * bytes)
+          dst[i0 + u * kBandThr] = v[u];
     }
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  for (int i = tid; i < a.T * nzpad; i += blockDim.x) {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int FMT, int NB>
+__global__ void __launch_bounds__(kBandThr, 3) band_dft_fp32_kernel(BandArgs a, int KG, int nzpad, int unit, int vec) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  constexpr int num = FmtBytes<FMT>::num, den = FmtBytes<FMT>::den;
+  const int     w       = blockIdx.y;
+  const int     tile_px = kBandThr * kBandPX / KG, bytes = tile_px * num / den;
+  uint8_t *stage = smem;                                                        // [2][T][bytes]
+  float2  *w_sh  = reinterpret_cast<float2 *>(smem + 2 * (size_t)a.T * bytes);  // [T][nzpad]
+  float2  *dc    = w_sh + (size_t)a.T * nzpad;                                  // [nzpad] shift sum_t W
+  int64_t *foff  = reinterpret_cast<int64_t *>(dc + nzpad);                     // [T] frame offsets
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int t = tid; t < a.T; t += kBandThr)
+    foff[t] = a.ring.frame(w, t) - a.ring.base;
+  __syncthreads();
+  const int64_t ntiles = (a.P + tile_px - 1) / tile_px;
+  const auto    fetch  = [&](int64_t tile, int s) {
+    if (tile >= ntiles) {
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      return;
+    }
+    const int64_t p0 = tile * tile_px;
+    const int     np = (int)min((int64_t)tile_px, a.P - p0);
+    stage_tile(stage + (size_t)s * a.T * bytes, a.ring.base + p0 * num / den, foff, a.T, bytes, np * num / den, unit);
+  };
+  fetch(blockIdx.x, 0);
+  for (int i = tid; i < a.T * nzpad; i += kBandThr) {
     const int t = i / nzpad, k = i % nzpad;
     w_sh[i]     = k < a.nz ? wmat_entry(a, w, t, k) : make_float2(0.f, 0.f);
   }
-  if (a.lens != nullptr)
-    for (int i = tid; i < tile_px; i += blockDim.x)
-      lens[i] = (tile0 + i < a.P) ? a.lens[tile0 + i] : make_float2(1.f, 0.f);
   __syncthreads();
+  for (int k = tid; k < nzpad; k += kBandThr) {
+    double sr = 0.0, si = 0.0;
+    if (FmtBytes<FMT>::shift != 0.f)
+      for (int t = 0; t < a.T; ++t)
+        sr += (double)w_sh[t * nzpad + k].x, si += (double)w_sh[t * nzpad + k].y;
+    dc[k] = make_float2((float)(FmtBytes<FMT>::shift * sr), (float)(FmtBytes<FMT>::shift * si));
+  }
 
-  const int g    = tid % groups;
-  const int half = tid / groups;
-  const int64_t p0 = tile0 + (int64_t)g * kBandPX;
-  const bool active = half < kBandHalf && p0 < a.P;
-  const int r = (int)(p0 / a.W), c = (int)(p0 % a.W);
-  float2 *outw = a.out + (int64_t)w * a.out_win + (int64_t)(r + a.oy) * a.OW + (c + a.ox);
-
-  for (int kc = half * kBandNB; kc < a.nz; kc += kBandNB * kBandHalf) {
-    float2 acc[kBandNB][kBandPX];
+  const int kgi = warp % KG, g = (warp / KG) * 32 + lane; // bin group, 4-pixel group of the tile
+  int       s   = 0;
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, s ^= 1) {
+    fetch(tile + gridDim.x, s ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const uint8_t *rows = stage + (size_t)s * a.T * bytes;
+    const int64_t  p0   = tile * tile_px + (int64_t)g * kBandPX;
+    for (int kc = kgi * NB; kc < a.nz; kc += KG * NB) {
+      float2 acc[NB][kBandPX];
 #pragma unroll
-    for (int b = 0; b < kBandNB; ++b)
+      for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int p = 0; p < kBandPX; ++p)
-        acc[b][p] = make_float2(0.f, 0.f);
-    if (active) {
+        for (int p = 0; p < kBandPX; ++p)
+          acc[b][p] = make_float2(0.f, 0.f);
+      const float4 *wr = reinterpret_cast<const float4 *>(w_sh + kc);
 #pragma unroll 2
       for (int t = 0; t < a.T; ++t) {
         float x[kBandPX];
-        load8<FMT>(tile + t * row_words, g, x);
-        const float2 *wr = w_sh + t * nzpad + kc;
+        load4<FMT>(rows + t * bytes, g, x);
 #pragma unroll
-        for (int b = 0; b < kBandNB; ++b) {
-          const float2 wv = wr[b];
+        for (int b = 0; b < NB; b += 2) {
+          const float4 wv = wr[t * (nzpad / 2) + b / 2];
 #pragma unroll
           for (int p = 0; p < kBandPX; ++p) {
-            acc[b][p].x = fmaf(x[p], wv.x, acc[b][p].x);
-            acc[b][p].y = fmaf(x[p], wv.y, acc[b][p].y);
+            acc[b][p]     = cfma2(make_float2(x[p], x[p]), make_float2(wv.x, wv.y), acc[b][p]);
+            acc[b + 1][p] = cfma2(make_float2(x[p], x[p]), make_float2(wv.z, wv.w), acc[b + 1][p]);
           }
         }
       }
+      if (p0 >= a.P)
+        continue;
+      float2 L[kBandPX];
 #pragma unroll
-      for (int b = 0; b < kBandNB; ++b) {
+      for (int p = 0; p < kBandPX; ++p)
+        L[p] = a.lens != nullptr && p0 + p < a.P ? __ldg(a.lens + p0 + p) : make_float2(1.f, 0.f);
+      float2 *out = a.out + (int64_t)w * a.out_win + p0;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
         const int k = kc + b;
-        if (k < a.nz) {
-          float4 *dst = reinterpret_cast<float4 *>(outw + (int64_t)k * a.out_plane);
+        if (k >= a.nz)
+          break;
+        float2 v[kBandPX];
 #pragma unroll
-          for (int p = 0; p < kBandPX; p += 2) {
-            float2 v0 = cscale(acc[b][p], a.scale), v1 = cscale(acc[b][p + 1], a.scale);
-            if (a.lens != nullptr) {
-              v0 = cmul(v0, lens[g * kBandPX + p]);
-              v1 = cmul(v1, lens[g * kBandPX + p + 1]);
-            }
-            dst[p / 2] = make_float4(v0.x, v0.y, v1.x, v1.y);
-          }
+        for (int p = 0; p < kBandPX; ++p) {
+          v[p] = cscale(cadd(acc[b][p], dc[k]), a.scale);
+          if (a.lens != nullptr)
+            v[p] = cmul(v[p], L[p]);
+        }
+        float2 *o = out + (int64_t)k * a.out_plane;
+        if (vec && p0 + kBandPX <= a.P) {
+          reinterpret_cast<float4 *>(o)[0] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+          reinterpret_cast<float4 *>(o)[1] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+        } else {
+#pragma unroll
+          for (int p = 0; p < kBandPX; ++p)
+            if (p0 + p < a.P)
+              o[p] = v[p];
         }
       }
     }
+    __syncthreads(); // this tile's rows are read: the stage takes the tile after next
   }
 }
 
@@ -168,8 +217,7 @@ template <int FMT> __global__ void band_dft_simple_kernel(BandArgs a) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= a.P)
     return;
-  const int r = (int)(p / a.W), c = (int)(p % a.W);
-  float2 *outp = a.out + (int64_t)w * a.out_win + (int64_t)(r + a.oy) * a.OW + (c + a.ox);
+  float2      *outp = a.out + (int64_t)w * a.out_win + p;
   const float2 L = a.lens ? a.lens[p] : make_float2(1.f, 0.f);
   for (int k0 = 0; k0 < a.nz; k0 += 8) {
     float2 acc[8];
@@ -199,26 +247,52 @@ template <int FMT> __global__ void band_dft_simple_kernel(BandArgs a) {
   }
 }
 
-template <int FMT> size_t tiled_smem(const BandArgs &a, int tile_px) {
-  const int nzpad = ((a.nz + kBandNB * kBandHalf - 1) / (kBandNB * kBandHalf)) * kBandNB * kBandHalf;
-  return (size_t)a.T * (tile_px * FmtBytes<FMT>::num / FmtBytes<FMT>::den) +
-         (size_t)a.T * nzpad * sizeof(float2) + (size_t)tile_px * sizeof(float2);
+// Bins per thread (even, at most 14), bin groups side by side, and shared memory of a launch.
+struct BandGeom {
+  int    NB, KG, nzpad;
+  size_t smem;
+};
+
+template <int FMT> BandGeom band_geom(int T, int nz) {
+  const int k  = (nz + 13) / 14; // bin groups
+  BandGeom  g{};
+  g.NB = std::max(4, ((nz + k - 1) / k + 1) / 2 * 2);
+  // the fewest groups side by side (the largest tile) that leave three CTAs per SM, else the most
+  for (g.KG = 1;; g.KG *= 2) {
+    g.nzpad = (nz + g.KG * g.NB - 1) / (g.KG * g.NB) * g.KG * g.NB;
+    g.smem  = 2 * (size_t)T * (kBandThr * kBandPX / g.KG) * FmtBytes<FMT>::num / FmtBytes<FMT>::den +
+             (size_t)(T + 1) * g.nzpad * sizeof(float2) + (size_t)T * sizeof(int64_t);
+    if (g.KG == 4 || g.smem <= 74 * 1024)
+      return g;
+  }
 }
 
-template <int FMT> int launch_tiled(const BandArgs &a, int nwin, cudaStream_t s) {
-  int tile_px = 1024;
-  while (tile_px > 128 && tiled_smem<FMT>(a, tile_px) > 110 * 1024)
-    tile_px /= 2;
-  const size_t smem = tiled_smem<FMT>(a, tile_px);
-  if (smem > 200 * 1024)
-    return HF_ERR_UNSUPPORTED;
-  HF_CUDA(cudaFuncSetAttribute(band_dft_tiled_kernel<FMT>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)((a.P + tile_px - 1) / tile_px), nwin);
-  const int threads = (tile_px / kBandPX) * kBandHalf;
-  band_dft_tiled_kernel<FMT><<<grid, threads, smem, s>>>(a, tile_px);
+template <int FMT, int NB> int launch_nb(const BandArgs &a, const BandGeom &g, int unit, int vec, int nwin, cudaStream_t s) {
+  HF_CUDA(cudaFuncSetAttribute(band_dft_fp32_kernel<FMT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+  const int     tile_px = kBandThr * kBandPX / g.KG;
+  const int64_t ntiles  = (a.P + tile_px - 1) / tile_px;
+  const int     per_sm  = std::max(1, std::min(3, (int)(220 * 1024 / g.smem)));
+  const int64_t ctas    = std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)per_sm * sm_count() / nwin));
+  band_dft_fp32_kernel<FMT, NB><<<dim3((unsigned)ctas, nwin), kBandThr, g.smem, s>>>(a, g.KG, g.nzpad, unit, vec);
   note_launch();
-  return launch_status("band_dft_tiled_kernel");
+  return launch_status("band_dft_fp32_kernel");
+}
+
+template <int FMT> int launch_fp32(const BandArgs &a, int nwin, cudaStream_t s) {
+  const BandGeom g = band_geom<FMT>(a.T, a.nz);
+  if (g.smem > 220 * 1024)
+    return HF_ERR_UNSUPPORTED;
+  const uintptr_t rows = reinterpret_cast<uintptr_t>(a.ring.base) | (uintptr_t)a.ring.frame_bytes;
+  const int       unit = rows % 16 == 0 ? 16 : (rows % 4 == 0 ? 4 : 1);
+  const int       vec  = reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.out_plane % 2 == 0 && a.out_win % 2 == 0;
+  switch (g.NB) {
+  case 4: return launch_nb<FMT, 4>(a, g, unit, vec, nwin, s);
+  case 6: return launch_nb<FMT, 6>(a, g, unit, vec, nwin, s);
+  case 8: return launch_nb<FMT, 8>(a, g, unit, vec, nwin, s);
+  case 10: return launch_nb<FMT, 10>(a, g, unit, vec, nwin, s);
+  case 12: return launch_nb<FMT, 12>(a, g, unit, vec, nwin, s);
+  default: return launch_nb<FMT, 14>(a, g, unit, vec, nwin, s);
+  }
 }
 
 template <int FMT> int launch_simple(const BandArgs &a, int nwin, cudaStream_t s) {
@@ -232,21 +306,16 @@ template <int FMT> int launch_simple(const BandArgs &a, int nwin, cudaStream_t s
 
 int launch_band_dft(const BandArgs &a, int fmt, int nwin, cudaStream_t s) {
   HF_CHECK_ARG(a.T > 0 && a.P > 0 && a.nz > 0 && nwin > 0, "band_dft: empty problem");
-  const bool tiled_ok = (a.P % kBandPX == 0) && (a.W % kBandPX == 0) && ((a.OW * 8) % 16 == 0) &&
-                        (a.ox % 2 == 0) && (a.ring.frame_bytes % 4 == 0) &&
-                        (((uintptr_t)a.ring.base & 3) == 0); // 4-byte cp.async copies of frame words
-  if (tiled_ok) {
-    int rc = HF_ERR_UNSUPPORTED;
-    switch (fmt) {
-    case HF_MONO12P: rc = launch_tiled<HF_MONO12P>(a, nwin, s); break;
-    case HF_U16: rc = launch_tiled<HF_U16>(a, nwin, s); break;
-    case HF_U8: rc = launch_tiled<HF_U8>(a, nwin, s); break;
-    case HF_F32: rc = launch_tiled<HF_F32>(a, nwin, s); break;
-    default: break;
-    }
-    if (rc != HF_ERR_UNSUPPORTED)
-      return rc;
+  int rc = HF_ERR_UNSUPPORTED; // (windows whose samples or W exceed shared memory, and complex frames)
+  switch (fmt) {
+  case HF_MONO12P: rc = launch_fp32<HF_MONO12P>(a, nwin, s); break;
+  case HF_U16: rc = launch_fp32<HF_U16>(a, nwin, s); break;
+  case HF_U8: rc = launch_fp32<HF_U8>(a, nwin, s); break;
+  case HF_F32: rc = launch_fp32<HF_F32>(a, nwin, s); break;
+  default: break;
   }
+  if (rc != HF_ERR_UNSUPPORTED)
+    return rc;
   switch (fmt) {
   case HF_MONO12P: return launch_simple<HF_MONO12P>(a, nwin, s);
   case HF_U16: return launch_simple<HF_U16>(a, nwin, s);

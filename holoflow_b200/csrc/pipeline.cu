@@ -288,10 +288,10 @@ static int phase_band(hf_plan *p, const FrameRing &fr, int nwin, const float2 *w
     HF_TRY(p->raw_tc ? launch_band_rows_tc(br, d.input_dtype, s) : launch_band_seg_tc(br, d.input_dtype, s));
   } else {
     BandArgs ba{};
-    ba.ring = fr, ba.T = d.frames, ba.P = p->P, ba.H = d.height, ba.W = d.width, ba.nz = p->nz;
+    ba.ring = fr, ba.T = d.frames, ba.P = p->P, ba.nz = p->nz;
     ba.wmat = wmat, ba.wmat_stride = wstride, ba.z0 = d.z_begin;
     ba.lens = d.propagation == HF_PROP_FRESNEL && !p->filter2d && !p->af ? p->lens : nullptr;
-    ba.out = p->band, ba.OH = d.height, ba.OW = d.width, ba.oy = 0, ba.ox = 0;
+    ba.out = p->band;
     ba.out_plane = p->P, ba.out_win = win_px, ba.scale = 1.0f;
     HF_TRY(launch_band_dft(ba, d.input_dtype, nwin, s));
     *lens_fused = ba.lens != nullptr;
