@@ -369,11 +369,13 @@ int hf_as_exec(hf_as_plan *p, const void *in, void *out, hf_stream_t s) {
   cp.out_col  = 1;
   float2 *o = reinterpret_cast<float2 *>(out);
   if (p->fast) {
-    rp.out = o; // a warp reads its whole row before writing it back, so in == out is safe
-    HF_TRY(launch_row_pass(rp, 1, s));
     cp.in  = o;
     cp.out = o;
     cp.tf  = p->tf;
+    if (col_tf_supported(cp)) // the placement's empty rows are neither transformed nor stored
+      rp.rows_only = 1, cp.row_lo = rp.oy, cp.row_hi = rp.oy + p->H;
+    rp.out = o; // a warp reads its whole row before writing it back, so in == out is safe
+    HF_TRY(launch_row_pass(rp, 1, s));
     HF_TRY(launch_col_pass(cp, COL_TF_SANDWICH, nullptr, 1, s));
     RowPass ri{};
     ri.in = o, ri.in_real = 0, ri.in_plane = oplane, ri.in_row = p->OW, ri.in_col = 1;

@@ -438,7 +438,9 @@ int launch_rowmom_fast(const ColPass &a, const MomentSpec &m, int nwin, cudaStre
 
 int launch_row_pass(const RowPass &a, int nwin, cudaStream_t s) {
   HF_CHECK_ARG(a.N > 0 && a.H > 0 && a.nplanes > 0 && nwin > 0, "row pass: empty problem");
-  if (fft_fast_length(a.N)) {
+  if (row_ring_supported(a))
+    return launch_row_ring(a, nwin, s);
+  if (fft_fast_length(a.N)) { // real, strided or unaligned rows
     if (a.inverse) {
       HF_DISPATCH_N1(a.N, return (launch_row_fast<N1, true>(a, nwin, s)))
     } else {
@@ -456,7 +458,10 @@ int launch_row_pass(const RowPass &a, int nwin, cudaStream_t s) {
   return launch_status("row_dft_generic_kernel");
 }
 
-int launch_col_pass(const ColPass &a, int mode, const MomentSpec *mom, int nwin, cudaStream_t s) {
+int launch_col_pass(const ColPass &pass, int mode, const MomentSpec *mom, int nwin, cudaStream_t s) {
+  ColPass a = pass;
+  if (a.row_hi == 0)
+    a.row_hi = a.H;
   HF_CHECK_ARG(a.H > 0 && a.W > 0 && a.nplanes > 0 && nwin > 0, "column pass: empty problem");
   MomentSpec m{};
   if (mom)
@@ -464,6 +469,11 @@ int launch_col_pass(const ColPass &a, int mode, const MomentSpec *mom, int nwin,
   if (mode == COL_MOMENTS)
     HF_CHECK_ARG(mom != nullptr && mom->nz == a.nplanes && a.nplanes <= kMaxBands,
                  "column moments: bad moment spec");
+  if (mode == COL_TF_SANDWICH) {
+    if (col_tf_supported(a))
+      return launch_col_tf(a, nwin, s);
+    HF_CHECK_ARG(a.row_lo == 0 && a.row_hi == a.H, "transfer-function columns: zero rows need the strip kernel");
+  }
   if (fft_fast_length(a.H)) {
     if (a.inverse) {
       HF_DISPATCH_N1(a.H, return (launch_col_fast<N1, true>(a, mode, m, nwin, s)))
@@ -487,6 +497,8 @@ int launch_col_pass(const ColPass &a, int mode, const MomentSpec *mom, int nwin,
 int launch_row_moments(const ColPass &a, const MomentSpec &m, int nwin, cudaStream_t s) {
   HF_CHECK_ARG(fft_fast_length(a.W), "row moments: unsupported row length");
   HF_CHECK_ARG(m.nz > 0 && m.nz <= kMaxBands, "row moments: bad moment spec");
+  if (row_moments_ring_supported(a))
+    return launch_row_moments_ring(a, m, nwin, s);
   if (a.inverse) {
     HF_DISPATCH_N1(a.W, return (launch_rowmom_fast<N1, true>(a, m, nwin, s)))
   } else {

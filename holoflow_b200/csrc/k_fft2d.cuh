@@ -42,6 +42,7 @@ struct RowPass {
   int           nplanes;       // planes per window
   const float2 *pre;           // optional [H][N] pre-multiply (applied to in-plane samples)
   int           inverse;
+  int           rows_only;     // 1: output rows outside the placed input need not be written
 };
 
 struct ColPass {
@@ -55,6 +56,8 @@ struct ColPass {
   const float2 *post;          // optional [H][W] post-multiply (complex store only)
   const float2 *tf;            // [H][W] transfer function (TF mode)
   int           inverse;
+  int           row_lo, row_hi; // TF mode: input rows outside [row_lo, row_hi) are zero, not
+                                // read (row_hi 0: every row is read; else col_tf_supported is needed)
 };
 
 enum ColMode { COL_COMPLEX = 0, COL_MAGNITUDE = 1, COL_MOMENTS = 2, COL_TF_SANDWICH = 3 };
@@ -63,6 +66,14 @@ enum ColMode { COL_COMPLEX = 0, COL_MAGNITUDE = 1, COL_MOMENTS = 2, COL_TF_SANDW
 bool fft_fast_length(int n);
 // Whether the any-length passes (k_fft_any.cu) cover transform length n.
 bool fft_any_length(int n);
+// The ring passes (k_rows_ring.cu) and the transfer-function columns (k_cols_tf.cu) by geometry and
+// alignment; launch_row_pass, launch_row_moments and launch_col_pass choose them.
+bool row_ring_supported(const RowPass &a);
+int  launch_row_ring(const RowPass &a, int nwin, cudaStream_t s);
+bool row_moments_ring_supported(const ColPass &a);
+int  launch_row_moments_ring(const ColPass &a, const MomentSpec &m, int nwin, cudaStream_t s);
+bool col_tf_supported(const ColPass &a);
+int  launch_col_tf(const ColPass &a, int nwin, cudaStream_t s);
 int  launch_row_any(const RowPass &a, int nwin, cudaStream_t s);
 int  launch_col_any(const ColPass &a, int magnitude, int nwin, cudaStream_t s);
 

@@ -425,14 +425,16 @@ static int phase_after_band(hf_plan *p, int nwin, float *out, cudaStream_t s, bo
   rp.IH = d.height, rp.IW = d.width, rp.oy = (p->OH - d.height) / 2, rp.ox = (p->OW - d.width) / 2;
   rp.H = p->OH, rp.N = p->OW, rp.nplanes = p->nz, rp.inverse = 0;
   rp.out = p->band2, rp.out_win = (int64_t)p->nz * oplane, rp.out_plane = oplane, rp.out_row = p->OW;
-  rec = p->timer.begin(s, ST_ROWS);
-  HF_TRY(launch_row_pass(rp, nwin, s));
-  p->timer.end(s, rec);
   ColPass cp{};
   cp.in = p->band2, cp.in_win = rp.out_win, cp.in_plane = oplane, cp.in_row = p->OW;
   cp.H = p->OH, cp.W = p->OW, cp.nplanes = p->nz;
   cp.out = p->band2, cp.out_win = rp.out_win, cp.out_plane = oplane, cp.out_row = p->OW, cp.out_col = 1;
   cp.tf = p->tf, cp.inverse = 0;
+  if (col_tf_supported(cp)) // the placement's empty rows are neither transformed nor stored
+    rp.rows_only = 1, cp.row_lo = rp.oy, cp.row_hi = rp.oy + d.height;
+  rec = p->timer.begin(s, ST_ROWS);
+  HF_TRY(launch_row_pass(rp, nwin, s));
+  p->timer.end(s, rec);
   rec = p->timer.begin(s, ST_COLS_TF);
   HF_TRY(launch_col_pass(cp, COL_TF_SANDWICH, nullptr, nwin, s));
   p->timer.end(s, rec);
