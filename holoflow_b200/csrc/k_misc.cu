@@ -4,6 +4,9 @@
 // as written in the reference kernels).
 #include <math_constants.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "k_misc.cuh"
 
 namespace hf {
@@ -78,37 +81,65 @@ __global__ void minmax_init_kernel(unsigned int *mm) {
   mm[1] = 0u;          // max
 }
 
-__global__ void minmax_kernel(const float *in, int64_t n, unsigned int *mm) {
-  unsigned int lo = 0xFFFFFFFFu, hi = 0u;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned int e = f2ord(in[i]);
-    lo                   = min(lo, e);
-    hi                   = max(hi, e);
+// One pair of atomics per CTA (a pair per warp of one-element threads serialised on the two words:
+// 44 us for 1024^2 values).
+__global__ void __launch_bounds__(256) minmax_kernel(const float *in, int64_t n, unsigned int *mm) {
+  unsigned int  lo = 0xFFFFFFFFu, hi = 0u;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = 4; // loads in flight per thread
+  int64_t       i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + (U - 1) * stride < n; i += U * stride) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      v[u] = in[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      lo = min(lo, f2ord(v[u])), hi = max(hi, f2ord(v[u]));
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
-    hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMin(mm, lo);
-    atomicMax(mm + 1, hi);
+  for (; i < n; i += stride)
+    lo = min(lo, f2ord(in[i])), hi = max(hi, f2ord(in[i]));
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  __shared__ unsigned int s[2][8];
+  if ((threadIdx.x & 31) == 0)
+    s[0][threadIdx.x >> 5] = lo, s[1][threadIdx.x >> 5] = hi;
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    lo = __reduce_min_sync(0xFFu, s[0][threadIdx.x]);
+    hi = __reduce_max_sync(0xFFu, s[1][threadIdx.x]);
+    if (threadIdx.x == 0) {
+      atomicMin(mm, lo);
+      atomicMax(mm + 1, hi);
+    }
   }
 }
 
-template <int TOP>
+// V consecutive values per thread (one 16-byte load and one 4- or 8-byte store when V = 4).
+template <int TOP, int V>
 __global__ void f32_scaled_kernel(const float *in, void *out, int64_t n, const unsigned int *mm) {
+  using T = typename std::conditional<TOP == 255, uint8_t, uint16_t>::type;
+  struct alignas(V * sizeof(T)) Out { T v[V]; };
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
+  if (i * V >= n)
     return;
   const float mn = ord2f(mm[0]), mx = ord2f(mm[1]);
   const float scale = __fdiv_rn((float)TOP, __fsub_rn(mx, mn));
-  const int   val   = (int)__fadd_rn(__fmul_rn(__fsub_rn(in[i], mn), scale), 0.5f);
-  const float cl    = fminf(fmaxf((float)val, 0.f), (float)TOP);
-  if constexpr (TOP == 255)
-    reinterpret_cast<uint8_t *>(out)[i] = (uint8_t)cl;
-  else
-    reinterpret_cast<uint16_t *>(out)[i] = (uint16_t)cl;
+  float       x[V];
+  if constexpr (V == 4) {
+    const float4 v = reinterpret_cast<const float4 *>(in)[i];
+    x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+  } else {
+    x[0] = in[i];
+  }
+  Out o;
+#pragma unroll
+  for (int u = 0; u < V; ++u) {
+    const int   val = (int)__fadd_rn(__fmul_rn(__fsub_rn(x[u], mn), scale), 0.5f);
+    const float cl  = fminf(fmaxf((float)val, 0.f), (float)TOP);
+    o.v[u]          = (T)cl;
+  }
+  reinterpret_cast<Out *>(out)[i] = o;
 }
 
 template <typename TI, int MODE> // MODE 0: real->F32, 1: real->CF32, 2: modulus, 3: argument
@@ -325,11 +356,17 @@ int launch_convert(const void *in, int in_dtype, void *out, int out_dtype, int s
     HF_CHECK_ARG(minmax_ws != nullptr, "Conversion: Scaled needs the min/max scratch");
     unsigned int *mm = reinterpret_cast<unsigned int *>(minmax_ws);
     minmax_init_kernel<<<1, 1, 0, s>>>(mm);
-    minmax_kernel<<<blocks_for(n, 256), 256, 0, s>>>((const float *)in, n, mm);
-    if (out_dtype == HF_U8)
-      f32_scaled_kernel<255><<<b, 256, 0, s>>>((const float *)in, out, n, mm);
+    minmax_kernel<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 4 * sm_count()), 256, 0, s>>>((const float *)in, n, mm);
+    const bool     v4 = n % 4 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % (out_dtype == HF_U8 ? 4 : 8) == 0;
+    const unsigned b4 = (unsigned)((n / 4 + 255) / 256);
+    if (out_dtype == HF_U8 && v4)
+      f32_scaled_kernel<255, 4><<<b4, 256, 0, s>>>((const float *)in, out, n, mm);
+    else if (out_dtype == HF_U8)
+      f32_scaled_kernel<255, 1><<<b, 256, 0, s>>>((const float *)in, out, n, mm);
+    else if (v4)
+      f32_scaled_kernel<65535, 4><<<b4, 256, 0, s>>>((const float *)in, out, n, mm);
     else
-      f32_scaled_kernel<65535><<<b, 256, 0, s>>>((const float *)in, out, n, mm);
+      f32_scaled_kernel<65535, 1><<<b, 256, 0, s>>>((const float *)in, out, n, mm);
     note_launch(2);
   } else {
     return fail(HF_ERR_INVALID, "Conversion: unknown strategy");

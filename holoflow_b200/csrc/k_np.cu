@@ -15,16 +15,19 @@ int np_blocks(int64_t n) {
 }
 
 // dst element i (row-major over `shape`) <- src at sum_d coord_d * src_strides_d bytes, written at
-// sum_d coord_d * dst_strides_d bytes.
-template <typename E> __global__ void copy_strided_kernel(const uint8_t *src, uint8_t *dst, NpLayout l, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rem = i, so = 0, doff = 0;
-    for (int d = l.rank - 1; d >= 0; --d) {
-      const int64_t c = rem % l.shape[d];
-      rem /= l.shape[d];
-      so += c * l.src_strides[d];
-      doff += c * l.dst_strides[d];
+// sum_d coord_d * dst_strides_d bytes.  I: index type (32 bits wherever the element count allows it).
+template <typename E, typename I> __global__ void copy_strided_kernel(const uint8_t *src, uint8_t *dst, NpLayout l, I n) {
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
+    I       rem = i;
+    int64_t so = 0, doff = 0;
+    for (int d = l.rank - 1; d > 0; --d) {
+      const I q = rem / (I)l.shape[d], c = rem - q * (I)l.shape[d];
+      rem = q;
+      so += (int64_t)c * l.src_strides[d];
+      doff += (int64_t)c * l.dst_strides[d];
     }
+    so += (int64_t)rem * l.src_strides[0];
+    doff += (int64_t)rem * l.dst_strides[0];
     *reinterpret_cast<E *>(dst + doff) = *reinterpret_cast<const E *>(src + so);
   }
 }
@@ -89,20 +92,68 @@ __global__ void causal_avg_kernel(const float *in, float *out, float *hist, floa
 
 } // namespace
 
-int launch_copy_strided(const void *src, void *dst, const NpLayout &l, int elem_size, cudaStream_t s) {
-  int64_t n = 1;
+namespace {
+// Dimensions that are contiguous with their inner neighbour in both tensors become one, and the
+// innermost contiguous run is copied in the widest elements that divide its length, its strides and
+// both addresses (a Slice of whole planes: one division per 16 bytes instead of four 64-bit ones per
+// element; 48 us for 42 MB of [2, 10 of 17, 512, 512] complex values before).
+int collapse_layout(NpLayout &l, int elem, const void *src, const void *dst) {
+  NpLayout c{};
+  for (int d = 0; d < l.rank; ++d) { // drop unit dimensions, merge from the outside in
+    if (l.shape[d] == 1)
+      continue;
+    const int q = c.rank - 1;
+    if (q >= 0 && c.src_strides[q] == l.shape[d] * l.src_strides[d] && c.dst_strides[q] == l.shape[d] * l.dst_strides[d]) {
+      c.shape[q] *= l.shape[d];
+      c.src_strides[q] = l.src_strides[d], c.dst_strides[q] = l.dst_strides[d];
+    } else {
+      c.shape[c.rank] = l.shape[d], c.src_strides[c.rank] = l.src_strides[d], c.dst_strides[c.rank] = l.dst_strides[d];
+      ++c.rank;
+    }
+  }
+  if (c.rank == 0)
+    c.rank = 1, c.shape[0] = 1, c.src_strides[0] = c.dst_strides[0] = elem;
+  const int in = c.rank - 1;
+  int       wide = elem;
+  if (c.src_strides[in] == elem && c.dst_strides[in] == elem) {
+    uint64_t all = (uint64_t)(c.shape[in] * elem) | reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
+    for (int d = 0; d < in; ++d)
+      all |= (uint64_t)c.src_strides[d] | (uint64_t)c.dst_strides[d];
+    while (wide < 16 && all % (2 * (uint64_t)wide) == 0)
+      wide *= 2;
+    c.shape[in] = c.shape[in] * elem / wide;
+    c.src_strides[in] = c.dst_strides[in] = wide;
+  }
+  l = c;
+  return wide;
+}
+
+template <typename E> void copy_strided(const uint8_t *a, uint8_t *b, const NpLayout &l, int64_t n, cudaStream_t s) {
+  if (n < (1ll << 31))
+    copy_strided_kernel<E, uint32_t><<<np_blocks(n), 256, 0, s>>>(a, b, l, (uint32_t)n);
+  else
+    copy_strided_kernel<E, int64_t><<<np_blocks(n), 256, 0, s>>>(a, b, l, n);
+}
+} // namespace
+
+int launch_copy_strided(const void *src, void *dst, const NpLayout &layout, int elem_size, cudaStream_t s) {
+  HF_CHECK_ARG(elem_size == 1 || elem_size == 2 || elem_size == 4 || elem_size == 8,
+               "strided copy: element size must be 1, 2, 4 or 8");
+  NpLayout  l    = layout;
+  const int wide = collapse_layout(l, elem_size, src, dst);
+  int64_t   n    = 1;
   for (int d = 0; d < l.rank; ++d)
     n *= l.shape[d];
   if (n == 0)
     return HF_OK;
   const auto *a = reinterpret_cast<const uint8_t *>(src);
   auto       *b = reinterpret_cast<uint8_t *>(dst);
-  switch (elem_size) {
-  case 1: copy_strided_kernel<uint8_t><<<np_blocks(n), 256, 0, s>>>(a, b, l, n); break;
-  case 2: copy_strided_kernel<uint16_t><<<np_blocks(n), 256, 0, s>>>(a, b, l, n); break;
-  case 4: copy_strided_kernel<uint32_t><<<np_blocks(n), 256, 0, s>>>(a, b, l, n); break;
-  case 8: copy_strided_kernel<uint2><<<np_blocks(n), 256, 0, s>>>(a, b, l, n); break;
-  default: return fail(HF_ERR_INVALID, "strided copy: element size must be 1, 2, 4 or 8");
+  switch (wide) {
+  case 1: copy_strided<uint8_t>(a, b, l, n, s); break;
+  case 2: copy_strided<uint16_t>(a, b, l, n, s); break;
+  case 4: copy_strided<uint32_t>(a, b, l, n, s); break;
+  case 8: copy_strided<uint2>(a, b, l, n, s); break;
+  default: copy_strided<uint4>(a, b, l, n, s); break;
   }
   note_launch();
   return launch_status("copy_strided_kernel");

@@ -20,7 +20,7 @@
 //  - hf_pctclip follows holotask/src/syncs/pct_clip.cu: the values at ranks
 //    int(p / 100 (count - 1)) of the pixels inside the ellipse (all slices), then
 //    min(max(x, lo), hi) on every pixel.  Instead of a full radix sort, an exact radix select:
-//    four passes of 8-bit shared-memory histograms over the same order-preserving float key
+//    three passes of 11-bit shared-memory histograms over the same order-preserving float key
 //    (sign bit set for positives, all bits inverted for negatives) find both ranks at once.
 #include <algorithm>
 #include <cmath>
@@ -45,17 +45,17 @@ struct ShiftGeom {
   int64_t shape[kShiftMaxDim], stride[kShiftMaxDim], shift[kShiftMaxDim]; // strides in elements
 };
 
-template <typename E>
-__global__ void fftshift_kernel(const E *__restrict__ in, E *__restrict__ out, ShiftGeom g, int64_t total) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rem = i, src = 0;
+template <typename E, typename I> // I: index type
+__global__ void fftshift_kernel(const E *__restrict__ in, E *__restrict__ out, ShiftGeom g, I total) {
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I rem = i, src = 0;
     for (int k = 0; k < g.ndim; ++k) {
-      const int64_t o = rem / g.stride[k];
-      rem -= o * g.stride[k];
-      int64_t s = o + g.shift[k];
-      if (s >= g.shape[k])
-        s -= g.shape[k];
-      src += s * g.stride[k];
+      const I st = (I)g.stride[k], o = rem / st;
+      rem -= o * st;
+      I s = o + (I)g.shift[k];
+      if (s >= (I)g.shape[k])
+        s -= (I)g.shape[k];
+      src += s * st;
     }
     out[i] = in[src];
   }
@@ -75,14 +75,19 @@ struct Taps {
   int   r;
   float w[2 * kFfMaxRadius + 1];
 };
-constexpr int kFfRowTile = 256;
-constexpr int kFfColTile = 64; // output rows per vertical tile (32 columns, 8 warps x 8 rows)
+constexpr int kFfRowThr  = 128;           // threads of a horizontal tile, 4 consecutive outputs each
+constexpr int kFfRowTile = 4 * kFfRowThr;
+constexpr int kFfColOut  = 8;             // consecutive output rows per thread of a vertical tile
+constexpr int kFfColTile = 8 * kFfColOut; // (32 columns x 8 threads)
+
+// Both passes keep a window of samples in registers, so a tap costs one shared-memory read per thread
+// instead of one per output; every output still sums its taps in ascending order, one fused
+// multiply-add each.
 
 // temp = horizontal Gaussian of each row (clamped at the row ends)
-__global__ void __launch_bounds__(kFfRowTile) flatfield_rows_kernel(const float *__restrict__ in,
-                                                                    float *__restrict__ tmp, int H, int W,
-                                                                    Taps t) {
-  __shared__ float tile[kFfRowTile + 2 * kFfMaxRadius];
+__global__ void __launch_bounds__(kFfRowThr) flatfield_rows_kernel(const float *__restrict__ in,
+                                                                   float *__restrict__ tmp, int H, int W, Taps t) {
+  __shared__ __align__(16) float tile[kFfRowTile + 2 * kFfMaxRadius + 6];
   const int64_t plane = (int64_t)blockIdx.z * H * W;
   const int     y = blockIdx.y, x0 = blockIdx.x * kFfRowTile;
   const float  *row = in + plane + (int64_t)y * W;
@@ -91,13 +96,33 @@ __global__ void __launch_bounds__(kFfRowTile) flatfield_rows_kernel(const float 
     tile[j]     = row[x];
   }
   __syncthreads();
-  const int x = x0 + threadIdx.x;
+  const int x = x0 + 4 * threadIdx.x;
   if (x >= W)
     return;
-  float sum = 0.f;
-  for (int k = 0; k <= 2 * t.r; ++k)
-    sum = fmaf(tile[threadIdx.x + k], t.w[k], sum);
-  tmp[plane + (int64_t)y * W + x] = sum;
+  const float4 *tp = reinterpret_cast<const float4 *>(tile) + threadIdx.x;
+  float         sum[4] = {0.f, 0.f, 0.f, 0.f};
+  float4        lo = tp[0];
+  const int     n = 2 * t.r + 1;
+  for (int k = 0; k < n; k += 4) { // taps k .. k + 3 on samples k .. k + 6 (the tile's tail is slack)
+    const float4 hi    = tp[k / 4 + 1];
+    const float  v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u < n)
+#pragma unroll
+        for (int o = 0; o < 4; ++o)
+          sum[o] = fmaf(v[u + o], t.w[k + u], sum[o]);
+    lo = hi;
+  }
+  float *dst = tmp + plane + (int64_t)y * W + x;
+  if (x + 4 <= W && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+    *reinterpret_cast<float4 *>(dst) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+  } else {
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+      if (x + o < W)
+        dst[o] = sum[o];
+  }
 }
 
 // out = in - vertical Gaussian of temp (clamped at the column ends)
@@ -113,17 +138,30 @@ __global__ void __launch_bounds__(256) flatfield_cols_kernel(const float *__rest
     tile[j][threadIdx.x] = tmp[plane + (int64_t)y * W + xc];
   }
   __syncthreads();
-  if (x >= W)
+  const int m0 = threadIdx.y * kFfColOut, n = 2 * t.r + 1;
+  if (x >= W || y0 + m0 >= H)
     return;
-  for (int m = threadIdx.y; m < kFfColTile; m += blockDim.y) {
-    const int y = y0 + m;
-    if (y >= H)
-      break;
-    float bg = 0.f;
-    for (int k = 0; k <= 2 * t.r; ++k)
-      bg = fmaf(tile[m + k][threadIdx.x], t.w[k], bg);
-    const int64_t i = plane + (int64_t)y * W + x;
-    out[i]          = in[i] - bg;
+  float bg[kFfColOut], v[kFfColOut]; // v: samples k .. k + 7 of the window, rotating
+#pragma unroll
+  for (int o = 0; o < kFfColOut; ++o)
+    bg[o] = 0.f, v[o] = o + 1 < kFfColOut ? tile[m0 + o][threadIdx.x] : 0.f;
+  for (int k = 0; k < n; k += kFfColOut) {
+#pragma unroll
+    for (int u = 0; u < kFfColOut; ++u)
+      if (k + u < n) {
+        v[(u + kFfColOut - 1) % kFfColOut] = tile[m0 + k + u + kFfColOut - 1][threadIdx.x];
+#pragma unroll
+        for (int o = 0; o < kFfColOut; ++o)
+          bg[o] = fmaf(v[(u + o) % kFfColOut], t.w[k + u], bg[o]);
+      }
+  }
+#pragma unroll
+  for (int o = 0; o < kFfColOut; ++o) {
+    const int y = y0 + m0 + o;
+    if (y < H) {
+      const int64_t i = plane + (int64_t)y * W + x;
+      out[i]          = in[i] - bg[o];
+    }
   }
 }
 
@@ -193,9 +231,13 @@ __global__ void filter2d_table_kernel(float2 *tab, int W, int H, uint32_t ri, ui
 // ------------------------------------------------------------------------------------------------
 // percentile clip
 // ------------------------------------------------------------------------------------------------
+// Radix select of the two ranks over the order-preserving key, 11 + 11 + 10 bits.  Between calls the
+// histograms and the ticket are zero: the CTA that finishes a pass last takes its step and clears them.
+constexpr int kSelBits = 11, kSelBins = 1 << kSelBits, kSelPasses = 3;
 struct SelState {
   uint32_t prefix[2], rank[2];
-  uint32_t hist[2][256];
+  uint32_t hist[2][kSelBins];
+  uint32_t ticket;
   float    lo, hi;
 };
 
@@ -231,73 +273,116 @@ __global__ void roi_mask_kernel(uint8_t *mask, int *count, int W, int H, int D, 
     atomicAdd(count, 1);
 }
 
-__global__ void select_init_kernel(SelState *st, uint32_t rank_lo, uint32_t rank_hi) {
-  for (int i = threadIdx.x; i < 512; i += blockDim.x)
-    (&st->hist[0][0])[i] = 0u;
-  if (threadIdx.x == 0) {
-    st->prefix[0] = st->prefix[1] = 0u;
-    st->rank[0] = rank_lo, st->rank[1] = rank_hi;
-  }
-}
-
-__global__ void __launch_bounds__(256) select_hist_kernel(const float *__restrict__ in, const uint8_t *__restrict__ mask,
-                                                          int64_t n, SelState *st, int pass) {
-  __shared__ uint32_t h[2][256];
-  for (int i = threadIdx.x; i < 512; i += blockDim.x)
+// One pass: digit histograms of the pixels that match each rank's prefix so far; the last CTA to
+// finish finds each rank's digit by a block-wide scan.  (One-thread scans in a launch of their own
+// took 11.6 us per pass, twice a pass over the image.)
+constexpr int kSelThr = 512;
+__global__ void __launch_bounds__(kSelThr) select_pass_kernel(const float *__restrict__ in,
+                                                              const uint8_t *__restrict__ mask, int64_t n, SelState *st,
+                                                              int pass, uint32_t rank_lo, uint32_t rank_hi) {
+  __shared__ uint32_t h[2][kSelBins];
+  __shared__ uint32_t warp_sum[kSelThr / 32];
+  __shared__ bool     last;
+  for (int i = threadIdx.x; i < 2 * kSelBins; i += kSelThr)
     (&h[0][0])[i] = 0u;
   __syncthreads();
-  const int      shift   = 24 - 8 * pass;
-  const uint32_t hi_mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-  const uint32_t p0 = st->prefix[0] & hi_mask, p1 = st->prefix[1] & hi_mask;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (!mask[i])
-      continue;
-    const uint32_t k   = float_key(in[i]);
-    const uint32_t bin = (k >> shift) & 255u;
+  const int      shift   = pass == 0 ? 21 : (pass == 1 ? 10 : 0), bits = pass == 2 ? 10 : 11;
+  const uint32_t hi_mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + bits)), digit = (1u << bits) - 1u;
+  const uint32_t p0 = pass == 0 ? 0u : st->prefix[0], p1 = pass == 0 ? 0u : st->prefix[1];
+  const auto count = [&](float v) {
+    const uint32_t k = float_key(v), bin = (k >> shift) & digit;
     if ((k & hi_mask) == p0)
       atomicAdd(&h[0][bin], 1u);
     if ((k & hi_mask) == p1)
       atomicAdd(&h[1][bin], 1u);
+  };
+  const int64_t stride = (int64_t)gridDim.x * kSelThr;
+  const bool    v4 = n % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0; // (the mask is 256-byte aligned)
+  if (v4) {
+    for (int64_t i = (int64_t)blockIdx.x * kSelThr + threadIdx.x; i < n / 4; i += stride) {
+      const uint32_t m = reinterpret_cast<const uint32_t *>(mask)[i];
+      if (m == 0u)
+        continue;
+      const float4 v = reinterpret_cast<const float4 *>(in)[i];
+      if (m & 0xFFu)
+        count(v.x);
+      if (m & 0xFF00u)
+        count(v.y);
+      if (m & 0xFF0000u)
+        count(v.z);
+      if (m >> 24)
+        count(v.w);
+    }
+  } else {
+    for (int64_t i = (int64_t)blockIdx.x * kSelThr + threadIdx.x; i < n; i += stride)
+      if (mask[i])
+        count(in[i]);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+  for (int i = threadIdx.x; i < 2 * kSelBins; i += kSelThr) {
     const uint32_t c = (&h[0][0])[i];
     if (c)
       atomicAdd(&(&st->hist[0][0])[i], c);
   }
-}
-
-__global__ void select_step_kernel(SelState *st, int pass) {
-  const int shift = 24 - 8 * pass;
-  if (threadIdx.x < 2) {
-    const int t   = threadIdx.x;
-    uint32_t  cum = 0, bin = 255;
-    for (uint32_t b = 0; b < 256; ++b) {
-      const uint32_t c = st->hist[t][b];
-      if (cum + c > st->rank[t]) {
-        bin = b;
-        break;
-      }
-      cum += c;
-    }
-    st->rank[t] -= cum;
-    st->prefix[t] |= bin << shift;
-    if (pass == 3) {
-      if (t == 0)
-        st->lo = key_float(st->prefix[0]);
-      else
-        st->hi = key_float(st->prefix[1]);
-    }
-  }
+  __threadfence();
   __syncthreads();
-  for (int i = threadIdx.x; i < 512; i += blockDim.x)
-    (&st->hist[0][0])[i] = 0u;
+  if (threadIdx.x == 0)
+    last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last)
+    return;
+  __threadfence();
+  // bins 4 i .. 4 i + 3 per thread; the digit is the bin whose cumulative range holds the rank
+  constexpr int B = kSelBins / kSelThr;
+  for (int t = 0; t < 2; ++t) {
+    volatile uint32_t *hist = st->hist[t];
+    const uint32_t     rank = pass == 0 ? (t == 0 ? rank_lo : rank_hi) : st->rank[t];
+    uint32_t           c[B], sum = 0u;
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      c[q] = hist[B * threadIdx.x + q], sum += c[q];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      incl += (threadIdx.x & 31) >= o ? u : 0u;
+    }
+    if ((threadIdx.x & 31) == 31)
+      warp_sum[threadIdx.x >> 5] = incl;
+    __syncthreads(); // (also: every thread has read st->rank[t])
+    uint32_t cum = incl - sum;
+    for (int q = 0; q < (int)(threadIdx.x >> 5); ++q)
+      cum += warp_sum[q];
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      if (rank >= cum && rank < cum + c[q]) { // exactly one bin of one thread
+        const uint32_t key = (pass == 0 ? 0u : st->prefix[t]) | (uint32_t)(B * threadIdx.x + q) << shift;
+        st->prefix[t] = key;
+        st->rank[t]   = rank - cum;
+        if (pass == kSelPasses - 1)
+          (t == 0 ? st->lo : st->hi) = key_float(key);
+      }
+      cum += c[q];
+      hist[B * threadIdx.x + q] = 0u;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0)
+    st->ticket = 0u;
 }
 
+template <bool V4>
 __global__ void clip_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t n, const SelState *st) {
   const float lo = st->lo, hi = st->hi;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = fminf(fmaxf(in[i], lo), hi);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (V4 ? n / 4 : n); i += (int64_t)gridDim.x * blockDim.x) {
+    if constexpr (V4) {
+      const float4 v = reinterpret_cast<const float4 *>(in)[i];
+      reinterpret_cast<float4 *>(out)[i] = make_float4(fminf(fmaxf(v.x, lo), hi), fminf(fmaxf(v.y, lo), hi),
+                                                       fminf(fmaxf(v.z, lo), hi), fminf(fmaxf(v.w, lo), hi));
+    } else {
+      out[i] = fminf(fmaxf(in[i], lo), hi);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -318,6 +403,14 @@ __global__ void slideavg_kernel(const float *__restrict__ x, float *__restrict__
 
 int grid_for(int64_t n, int block = 256) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + block - 1) / block, (int64_t)sm_count() * 16));
+}
+
+template <typename E> void launch_shift(const void *in, void *out, const ShiftGeom &g, int64_t total, cudaStream_t s) {
+  const int grid = grid_for(total);
+  if (total < (1ll << 31))
+    fftshift_kernel<E, uint32_t><<<grid, 256, 0, s>>>((const E *)in, (E *)out, g, (uint32_t)total);
+  else
+    fftshift_kernel<E, int64_t><<<grid, 256, 0, s>>>((const E *)in, (E *)out, g, total);
 }
 
 // std::to_string(float) keeps six decimals: the value the reference's JIT source compiles in
@@ -458,24 +551,40 @@ int hf_fftshift(const void *in, void *out, int elem_size, int ndim, const int64_
   HF_CHECK_ARG(elem_size == 1 || elem_size == 2 || elem_size == 3 || elem_size == 4 || elem_size == 8 ||
                    elem_size == 16,
                "FFTShift: element size must be 1, 2, 3, 4, 8 or 16 bytes");
-  ShiftGeom g{};
-  g.ndim        = ndim;
-  int64_t total = 1;
-  for (int k = ndim - 1; k >= 0; --k) {
+  // Runs of w elements that move together are shifted as one wider element (up to 16 bytes); axes that
+  // do not shift are merged with their inner neighbour.
+  int64_t inner = shape[ndim - 1], ishift = (axes_mask >> (ndim - 1)) & 1u ? inner / 2 : 0;
+  for (int k = 0; k < ndim; ++k)
     HF_CHECK_ARG(shape[k] > 0, "FFTShift: input tensor has zero elements");
-    g.shape[k]  = shape[k];
-    g.stride[k] = total;
-    g.shift[k]  = (axes_mask >> k) & 1u ? shape[k] / 2 : 0;
-    total *= shape[k];
+  int es = elem_size;
+  while (es < 16 && es != 3 && inner % 2 == 0 && ishift % 2 == 0 &&
+         ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & (2 * es - 1)) == 0)
+    es *= 2, inner /= 2, ishift /= 2;
+  ShiftGeom g{};
+  g.ndim  = 1;
+  int at  = kShiftMaxDim - 1; // dimensions are filled from the innermost outwards
+  g.shape[at] = inner, g.shift[at] = ishift;
+  for (int k = ndim - 2; k >= 0; --k) {
+    const int64_t sh = (axes_mask >> k) & 1u ? shape[k] / 2 : 0;
+    if (sh == 0 && g.shift[at] == 0) {
+      g.shape[at] *= shape[k];
+    } else {
+      --at, ++g.ndim;
+      g.shape[at] = shape[k], g.shift[at] = sh;
+    }
   }
-  const int grid = grid_for(total);
-  switch (elem_size) {
-  case 1: fftshift_kernel<uint8_t><<<grid, 256, 0, s>>>((const uint8_t *)in, (uint8_t *)out, g, total); break;
-  case 2: fftshift_kernel<uint16_t><<<grid, 256, 0, s>>>((const uint16_t *)in, (uint16_t *)out, g, total); break;
-  case 3: fftshift_kernel<Bytes3><<<grid, 256, 0, s>>>((const Bytes3 *)in, (Bytes3 *)out, g, total); break;
-  case 4: fftshift_kernel<uint32_t><<<grid, 256, 0, s>>>((const uint32_t *)in, (uint32_t *)out, g, total); break;
-  case 8: fftshift_kernel<uint2><<<grid, 256, 0, s>>>((const uint2 *)in, (uint2 *)out, g, total); break;
-  default: fftshift_kernel<Bytes16><<<grid, 256, 0, s>>>((const Bytes16 *)in, (Bytes16 *)out, g, total); break;
+  int64_t total = 1;
+  for (int k = 0; k < g.ndim; ++k)
+    g.shape[k] = g.shape[at + k], g.shift[k] = g.shift[at + k];
+  for (int k = g.ndim - 1; k >= 0; --k)
+    g.stride[k] = total, total *= g.shape[k];
+  switch (es) {
+  case 1: launch_shift<uint8_t>(in, out, g, total, s); break;
+  case 2: launch_shift<uint16_t>(in, out, g, total, s); break;
+  case 3: launch_shift<Bytes3>(in, out, g, total, s); break;
+  case 4: launch_shift<uint32_t>(in, out, g, total, s); break;
+  case 8: launch_shift<uint2>(in, out, g, total, s); break;
+  default: launch_shift<Bytes16>(in, out, g, total, s); break;
   }
   note_launch();
   return launch_status("fftshift_kernel");
@@ -549,7 +658,7 @@ int hf_flatfield_exec(hf_flatfield *f, const float *in, float *out, hf_stream_t 
   const int64_t P = (int64_t)H * W;
   if (!f->fourier) {
     HF_CHECK_ARG(f->planes <= 65535, "Flatfield: at most 65535 planes");
-    flatfield_rows_kernel<<<dim3((W + kFfRowTile - 1) / kFfRowTile, H, (unsigned)f->planes), kFfRowTile, 0, s>>>(
+    flatfield_rows_kernel<<<dim3((W + kFfRowTile - 1) / kFfRowTile, H, (unsigned)f->planes), kFfRowThr, 0, s>>>(
         in, f->tmp, H, W, f->tx);
     note_launch();
     HF_TRY(launch_status("flatfield_rows_kernel"));
@@ -644,6 +753,8 @@ int hf_pctclip_create(int depth, int height, int width, float min_pct, float max
   if (rc == HF_OK)
     rc = cuda_status(cudaMalloc(&p->st, sizeof(SelState)), "PctClip: state");
   if (rc == HF_OK)
+    rc = cuda_status(cudaMemsetAsync(p->st, 0, sizeof(SelState), s), "PctClip: state");
+  if (rc == HF_OK)
     rc = cuda_status(cudaMalloc(&cnt, sizeof(int)), "PctClip: count");
   if (rc == HF_OK)
     rc = cuda_status(cudaMemsetAsync(cnt, 0, sizeof(int), s), "PctClip: count");
@@ -683,17 +794,16 @@ int hf_pctclip_exec(hf_pctclip *p, const float *in, float *out, float *bounds, h
   clear_error();
   HF_CHECK_ARG(p != nullptr && in != nullptr && out != nullptr, "PctClip: null argument");
   const int64_t n = (int64_t)p->D * p->H * p->W;
-  select_init_kernel<<<1, 256, 0, s>>>(p->st, (uint32_t)p->min_idx, (uint32_t)p->max_idx);
-  note_launch();
-  HF_TRY(launch_status("select_init_kernel"));
-  const int grid = grid_for(n, 256 * 8);
-  for (int pass = 0; pass < 4; ++pass) {
-    select_hist_kernel<<<grid, 256, 0, s>>>(in, p->mask, n, p->st, pass);
-    select_step_kernel<<<1, 256, 0, s>>>(p->st, pass);
-    note_launch(2);
-    HF_TRY(launch_status("select_hist_kernel"));
+  const int grid = (int)std::min<int64_t>((n + 4 * kSelThr - 1) / (4 * kSelThr), sm_count());
+  for (int pass = 0; pass < kSelPasses; ++pass) {
+    select_pass_kernel<<<grid, kSelThr, 0, s>>>(in, p->mask, n, p->st, pass, (uint32_t)p->min_idx, (uint32_t)p->max_idx);
+    note_launch();
+    HF_TRY(launch_status("select_pass_kernel"));
   }
-  clip_kernel<<<grid_for(n), 256, 0, s>>>(in, out, n, p->st);
+  if (n % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+    clip_kernel<true><<<grid_for(n / 4), 256, 0, s>>>(in, out, n, p->st);
+  else
+    clip_kernel<false><<<grid_for(n), 256, 0, s>>>(in, out, n, p->st);
   note_launch();
   HF_TRY(launch_status("clip_kernel"));
   if (bounds)
