@@ -2,23 +2,32 @@
 //
 // The clutter filter W = (I - V_r V_r^T) D needs only the top clutter_rank eigenvectors of each
 // window's Gram matrix, and the full cyclic Jacobi solve (k_pca.cu) spends O(n^3) shared-memory
-// traffic per sweep over ~11 sweeps.  Here one CTA of 256 threads per matrix runs:
+// traffic per sweep over ~11 sweeps.  Here one CTA per matrix (128, 256 or 512 threads for n up to 32,
+// 64 or 128) runs:
 //  1. Householder reduction to tridiagonal form, A = Q T Q^T (Golub & Van Loan, Matrix
-//     Computations, 4th ed., Alg. 8.3.1), with the reflectors v_k kept in column k below the
-//     subdiagonal and beta_k in a side array.  Two barriers per step: the matrix-vector product
-//     p = beta A v (a thread pair per row, each summing half the row) with per-warp partials of
-//     p^T v; then the rank-2 update A -= v w^T + w v^T with w = p - (beta/2)(p^T v) v formed on the
-//     fly, where warp 0 updates the trailing block's first column and at once builds the next
-//     step's house vector from it (the house vectors alternate between two buffers);
-//  2. the r largest eigenvalues of T by Sturm-sequence multisection (Wilkinson): a warp evaluates
-//     32 shifts at once, each lane counting the sign changes of the leading-minor sequence
-//     p_j = (d_j - x) p_{j-1} - e_{j-1}^2 p_{j-2} (rescaled by powers of two, no division), and the
-//     bracket shrinks 33x per round;
-//  3. their eigenvectors of T by inverse iteration (Wilkinson): three solves with the tridiagonal
+//     Computations, 4th ed., Alg. 8.3.1), with the matrix in registers: a half-warp per four rows, a
+//     thread holding n / 16 columns of them.  Two barriers per step: p = beta A v (the four rows' sums
+//     are reduced and scattered over the half-warp together) with per-warp partials of p^T v; then the
+//     rank-2 update, after which the half-warp of row k + 1 builds the next house vector from its
+//     registers and writes it where the back-transformation reads it;
+//  2. the r largest eigenvalues of T by Sturm-sequence multisection (Wilkinson): a warp evaluates 32
+//     shifts at once and the bracket shrinks 33x per round (four chains per lane take 8 rounds for 11,
+//     but twice the time: the FP64 pipe takes a warp's instruction every two cycles);
+//  3. their eigenvectors of T by inverse iteration (Wilkinson): two solves with the tridiagonal
 //     LU factorisation of T - lambda I with partial pivoting, pivots floored at eps ||T||, from
 //     distinct starting vectors, orthonormalised (modified Gram-Schmidt) within clusters of close
 //     eigenvalues after each solve;
-//  4. back-transformation V_r = Q Y by the reflectors in reverse order, a warp per column.
+//  4. back-transformation V_r = Q Y by the reflectors in reverse order, four per step, a warp per
+//     column.
+// Bound: one CTA on one SM.  A step's vectors cross shared memory, whose 128 bytes per cycle every
+// thread shares: with four threads per row, each reading whole quarters of v and p, those reads alone
+// took 800 (n = 64) to 3000 (n = 128) cycles per step; 4 x (n / 16) tiles read a third of that.  The
+// rest is latency: dependent FP64 operations (9 cycles), shuffles, barriers.  So the library's square
+// root and two divisions per house vector became float-seeded third-order Newton steps (the matrix is
+// scaled to entries below 1), sums run pairwise, independent chains run side by side, values a chain
+// needs are loaded ahead of it, and finished rows and columns are skipped.
+// Measured, 8 matrices, r = 4, before -> now: n = 32 86 -> 50 us, 64 172 -> 99, 128 396 -> 254 (at n = 64:
+// reduction 51 us, eigenvalues 14, factors and inverse iteration 20, back-transformation 6).
 // The eigenvalues ascend in evals[n - r .. n - 1] and the vectors go to the matching columns of
 // evecs ([n][n], column = eigenvalue index, as the Jacobi solver lays them out); the other entries
 // are not written.  info = 0, or 1 when the input is not finite.
@@ -30,14 +39,15 @@ namespace hf {
 
 namespace {
 
-constexpr int kEigThr  = 256;
-constexpr int kEigWarps = kEigThr / 32;
 constexpr int kEigMaxN = 128;
 constexpr int kEigMaxR = 16;
+constexpr int kEigRed  = 20; // reduction slots (up to 16 warps)
 
 // Stride of the per-eigenvalue vectors, = 1 (mod 16) doubles, so the lanes of the inverse iteration
 // (one per eigenvalue, r <= 16) address distinct bank pairs.
 __host__ __device__ inline int eig_ldy(int n) { return 16 * ((n + 15) / 16) + 1; }
+// Threads of a CTA: a half-warp per four rows.
+__host__ __device__ inline int eig_threads(int n) { return n <= 32 ? 128 : (n <= 64 ? 256 : 512); }
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -46,199 +56,274 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Number of eigenvalues of the tridiagonal (d, e) below x: sign changes of the leading minors of
-// T - x I.  T is scaled by a power of two to ||T|| <= 1, so a minor grows at most 3x per step; two
-// steps at a time, consecutive minors are rescaled together by 2^-/+800 when they leave
-// [2^-800, 2^800], which keeps every sign.  A zero minor counts as a change.
-__device__ int sturm_count(const double *d, const double *e2, int n, double x) {
-  double pm = 1.0, p = d[0] - x;
-  int    cnt = p <= 0.0 ? 1 : 0; // p_0 = 1 > 0
-  if (p == 0.0)
-    p = -DBL_MIN; // counted; continue from a tiny negative minor
-  const auto step = [&](int j) {
-    double q = fma(d[j] - x, p, -e2[j - 1] * pm);
-    if (q == 0.0)
-      q = p > 0.0 ? -DBL_MIN : DBL_MIN;
-    cnt += (q < 0.0) != (p < 0.0);
-    pm = p;
-    p  = q;
-  };
-  int j = 1;
-  for (; j + 1 < n; j += 2) {
-    step(j);
-    step(j + 1);
-    const double a = fabs(p);
-    const double f = a > 0x1p800 ? 0x1p-800 : (a < 0x1p-800 && fabs(pm) < 0x1p-800 ? 0x1p800 : 1.0);
+// Number of eigenvalues of the tridiagonal (d, e) below x: sign changes of the leading minors
+// p_j = (d_j - x) p_(j-1) - e_(j-1)^2 p_(j-2) of T - x I.  T is scaled to ||T|| < 1, |d_j - x| is kept at
+// or above 2^-60 and e2 at or above 2^-120 (perturbations far below the rounding of T), so four steps
+// change a minor by less than 2^+-301 relative to the pair before them: the pair is rescaled by 2^+-300
+// between groups of four and no sign is lost.  Zero counts as positive: the minor after a zero has the
+// sign opposite to the one before it, so the pair still counts one change.
+__device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x) {
+  double p = d[0] - x, pm = 1.0;
+  int    cnt = (unsigned)__double2hiint(p) >> 31;
+  double dj[4], ej[4]; // (the arrays hold eight entries beyond n)
+#pragma unroll
+  for (int jj = 0; jj < 4; ++jj)
+    dj[jj] = d[1 + jj], ej[jj] = e2[jj];
+  for (int j0 = 1; j0 < n; j0 += 4) {
+    double dn[4], en[4]; // the next group's entries, loaded ahead of the chain
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj)
+      dn[jj] = d[j0 + 4 + jj], en[jj] = e2[j0 + 3 + jj];
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      double    dx = dj[jj] - x;
+      const int hi = __double2hiint(dx);
+      if ((hi & 0x7FFFFFFF) < 0x3C300000) // |dx| < 2^-60
+        dx = __hiloint2double((hi & 0x80000000) | 0x3C300000, 0);
+      const double q = fma(dx, p, -(ej[jj] * pm));
+      cnt += (unsigned)(__double2hiint(q) ^ __double2hiint(p)) >> 31;
+      pm = p;
+      p  = q;
+    }
+    // by the larger exponent: above 2^300 or below 2^-300
+    const int    ex = max(__double2hiint(p) & 0x7FF00000, __double2hiint(pm) & 0x7FF00000);
+    const double f =
+        __hiloint2double(ex > (1323 << 20) ? (723 << 20) : (ex < (723 << 20) ? (1323 << 20) : (1023 << 20)), 0);
     p *= f;
     pm *= f;
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj)
+      dj[jj] = dn[jj], ej[jj] = en[jj];
   }
-  if (j < n)
-    step(j);
   return cnt;
 }
 
-__global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, double *evecs, double *evals,
-                                                          int *info, int n, int r) {
+// Hardware approximations (relative error below 2^-21) that seed the Newton steps.
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// 1 / sqrt(t) and 1 / t for t in the normal float range, to double precision: a float32 seed
+// (relative error below 2^-21) and one third-order Newton step, e -> O(e^3).
+__device__ __forceinline__ double rsqrt_seeded(double t, float seed) {
+  const double y = (double)seed, a = t * y, e = fma(-a, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double rcp_seeded(double t, float seed) {
+  const double r = (double)seed, e = fma(-t, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+__device__ __forceinline__ double reciprocal(double x) {
+  return fabs(x) > 1e-30 && fabs(x) < 1e30 ? rcp_seeded(x, rcp_approx((float)x)) : 1.0 / x;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) eig_top_kernel(const double *a_in, double *evecs, double *evals, int *info,
+                                                        int n, int r) {
+  constexpr int kWarps = NT / 32;
+  constexpr int RM     = NT / 4;          // rows the CTA can hold
+  constexpr int M      = RM / 32;         // column pairs per thread: columns 2 tc, 2 tc + 1 (+ 32 m)
+  constexpr int NC     = RM / 32;         // entries of a vector per lane
   extern __shared__ __align__(16) double esm[];
-  const int ld   = n + 1;                 // padded row stride
-  double   *A    = esm;                   // [n][ld]
-  double   *beta = A + n * ld;            // [n]
+  double   *R    = esm;                   // [n][RM] house vectors, zero up to their own index
+  double   *pw   = R + n * RM;            // [RM] p = beta A v
+  double   *beta = pw + RM;               // [n]
   double   *d    = beta + n;              // [n] diagonal of T
   double   *e    = d + n;                 // [n] subdiagonal of T (e[n-1] = 0)
-  double   *e2   = e + n;                 // [n] e^2, scaled by sc^2
-  double   *ds   = e2 + n;                // [n] d, scaled by sc (||T|| sc <= 1)
-  double   *vvb  = ds + n;                // [2][n] house vectors of even / odd steps
-  double   *pw   = vvb + 2 * n;           // [n] p = beta A v
-  double   *lam  = pw + n;                // [kEigMaxR] eigenvalues, descending
+  double   *e2   = e + n;                 // [n + 8] e^2, scaled by sc^2
+  double   *ds   = e2 + n + 8;            // [n + 8] d, scaled by sc (||T|| sc <= 1)
+  double   *lam  = ds + n + 8;            // [kEigMaxR] eigenvalues, descending
   const int ldy  = eig_ldy(n);            // per-vector stride: lane t's entries in bank pair t
   double   *Y    = lam + kEigMaxR;        // [kEigMaxR][ldy] eigenvectors of T, then of A
   double   *lu   = Y + kEigMaxR * ldy;    // [4][kEigMaxR][ldy] LU factors of each shift
-  double   *red  = lu + 4 * kEigMaxR * ldy; // [kEigWarps + 4] reductions and scalars
-  int      *flag = reinterpret_cast<int *>(red + kEigWarps + 4);
+  double   *red  = lu + 4 * kEigMaxR * ldy; // [kEigRed] reductions and scalars
 
   const int     tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int     i0 = 4 * (tid >> 4), tc = lane & 15; // the half-warp's first row; this thread's columns
   const double *src = a_in + (int64_t)blockIdx.x * n * n;
-  if (tid == 0)
-    *flag = 0;
-  __syncthreads();
-  for (int x = tid; x < n * n; x += kEigThr) {
-    const int    i = x / n, j = x % n;
-    const double v = 0.5 * (src[i * n + j] + src[j * n + i]);
-    if (!isfinite(v))
-      *flag = 1;
-    A[i * ld + j] = v;
-  }
-  __syncthreads();
-  if (*flag) { // not finite: report, leave the outputs alone
+  double        a[4][2 * M], big = 0.0; // symmetric part, and its largest magnitude
+  bool          finite = true;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int c = 0; c < 2 * M; ++c) {
+      const int i = i0 + q, j = 2 * tc + (c & 1) + 32 * (c >> 1);
+      a[q][c]     = i < n && j < n ? 0.5 * (src[i * n + j] + src[j * n + i]) : 0.0;
+      finite      = finite && isfinite(a[q][c]);
+      big         = fmax(big, fabs(a[q][c]));
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0)
+    red[warp] = big;
+  if (__syncthreads_or(!finite)) { // not finite: report, leave the outputs alone
     if (tid == 0 && info != nullptr)
       info[blockIdx.x] = 1;
     return;
   }
+  // scale by a power of two to a largest entry in [1/2, 1): exact, and the house vectors' squared
+  // norms stay in the float range that seeds their square roots
+  big = red[0];
+#pragma unroll
+  for (int q = 1; q < kWarps; ++q)
+    big = fmax(big, red[q]);
+  int ex = 0;
+  frexp(big, &ex);
+  {
+    const double f1 = ldexp(1.0, -ex / 2), f2 = ldexp(1.0, -ex - (-ex / 2));
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int c = 0; c < 2 * M; ++c)
+        a[q][c] = a[q][c] * f1 * f2;
+  }
 
   // ---- 1. Householder tridiagonalisation ------------------------------------------------------
-  // house vector of step k from column k below the diagonal (warp 0); its reflector replaces the
-  // column's entries, beta_k, d_k and e_k go to their arrays
+  // House vector of step k by the half-warp of row k, from the entries x beyond the diagonal:
+  // v = x + sign(x_0) ||x|| e_0, beta = 2 / v^T v = 1 / (t + |x_0| ||x||) with t = ||x||^2.
   const auto house = [&](int k) {
-    const int m = n - k - 1;
-    double   *v = vvb + (k & 1) * n;
-    double    s = 0.0;
-    for (int i = 1 + lane; i < m; i += 32) {
-      const double x = A[(k + 1 + i) * ld + k];
-      s              = fma(x, x, s);
+    const unsigned half = 0xFFFFu << (lane & 16);
+    double         x[2 * M], sa = 0.0, sb = 0.0, xs = 0.0, xd = 0.0;
+#pragma unroll
+    for (int c = 0; c < 2 * M; ++c) {
+      const int j = 2 * tc + (c & 1) + 32 * (c >> 1);
+      x[c] = (k & 2) ? ((k & 1) ? a[3][c] : a[2][c]) : ((k & 1) ? a[1][c] : a[0][c]);
+      xs   = j == k + 1 ? x[c] : xs; // the owner of entry k + 1 / k
+      xd   = j == k ? x[c] : xd;
+      x[c] = j > k + 1 ? x[c] : 0.0;
+      if (c & 1)
+        sb = fma(x[c], x[c], sb);
+      else
+        sa = fma(x[c], x[c], sa);
     }
-    s               = warp_sum(s);
-    const double x0 = A[(k + 1) * ld + k];
-    double       v0 = 1.0, b = 0.0, alpha = x0;
+    const double x0 = __shfl_sync(half, xs, (lane & 16) + (((k + 1) & 31) >> 1));
+    double       s  = sa + sb;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+      s += __shfl_xor_sync(half, s, o);
+    double v0 = 0.0, b = 0.0, alpha = x0;
     if (s > 0.0) {
-      const double mu = sqrt(fma(x0, x0, s));
-      v0              = x0 <= 0.0 ? x0 - mu : -s / (x0 + mu); // x0 - mu without cancellation
-      b               = 2.0 / fma(v0, v0, s);
-      alpha           = mu;
+      const double t = fma(x0, x0, s);
+      double       mu;
+      if (t > 1e-30) { // t <= n: in the float range
+        const float tf = (float)t, yf = rsqrt_approx(tf);
+        mu = t * rsqrt_seeded(t, yf);
+        b  = rcp_seeded(fma(fabs(x0), mu, t), rcp_approx(fmaf(fabsf((float)x0), tf * yf, tf)));
+      } else {
+        mu = sqrt(t);
+        b  = 1.0 / fma(fabs(x0), mu, t);
+      }
+      if (isfinite(b)) { // (a norm whose square underflows leaves the row as it is: v = 0, H = I)
+        v0    = x0 + copysign(mu, x0);
+        alpha = -copysign(mu, x0);
+      } else {
+        b = 0.0;
+      }
     }
-    for (int i = lane; i < m; i += 32)
-      v[i] = i == 0 ? v0 : A[(k + 1 + i) * ld + k];
-    __syncwarp();
-    if (lane == 0) {
-      A[(k + 1) * ld + k] = v0;
-      beta[k]             = b;
-      d[k]                = A[k * ld + k];
-      e[k]                = alpha;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int j  = 2 * tc + 32 * m;
+      double2   vv = b != 0.0 ? make_double2(x[2 * m], x[2 * m + 1]) : make_double2(0.0, 0.0);
+      vv.x = j == k + 1 ? v0 : vv.x;
+      vv.y = j + 1 == k + 1 ? v0 : vv.y;
+      *reinterpret_cast<double2 *>(R + k * RM + j) = vv;
+    }
+    if (tc == ((k & 31) >> 1)) {
+      beta[k] = b;
+      d[k]    = xd;
+      e[k]    = alpha;
     }
   };
-  if (warp == 0 && n >= 3)
+  const int ip = i0 + ((lane >> 2) & 3); // the row whose p this lane ends up with
+  if (i0 == 0 && n >= 3)
     house(0);
   __syncthreads();
   for (int k = 0; k + 2 < n; ++k) {
-    const int     m = n - k - 1; // trailing block rows / cols k+1 .. n-1
-    const double  b = beta[k];
-    const double *v = vvb + (k & 1) * n;
-    if (b == 0.0) { // the column is already reduced: H = I, the trailing block stays
-      if (warp == 0 && k + 3 < n)
-        house(k + 1);
-      __syncthreads();
-      continue;
-    }
-    { // p = beta A' v: threads 2i and 2i+1 sum the two halves of row i (read as column i of the
-      // symmetric block, so a warp's loads are contiguous), then the warp's share of p^T v
-      const int i = tid >> 1, hm = (m + 1) >> 1;
-      double    s0 = 0.0, s1 = 0.0;
-      if (i < m) {
-        const int     j1  = min(m, (tid & 1) * hm + hm);
-        const double *col = A + (k + 1) * ld + k + 1 + i;
-        int           j   = (tid & 1) * hm;
-        double        s2 = 0.0, s3 = 0.0;
-        for (; j + 3 < j1; j += 4) {
-          s0 = fma(col[j * ld], v[j], s0);
-          s1 = fma(col[(j + 1) * ld], v[j + 1], s1);
-          s2 = fma(col[(j + 2) * ld], v[j + 2], s2);
-          s3 = fma(col[(j + 3) * ld], v[j + 3], s3);
-        }
-        for (; j < j1; ++j)
-          s0 = fma(col[j * ld], v[j], s0);
-        s0 += s2;
-        s1 += s3;
+    const double  b = beta[k], *v = R + k * RM;
+    const bool    live = 8 * warp + 7 > k; // the warp has unfinished rows
+    const double  vi = v[ip];
+    double        s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      if (live && 32 * m + 31 > k) { // v is zero up to entry k
+        const double2 vv = *reinterpret_cast<const double2 *>(v + 2 * tc + 32 * m);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          s[q] = fma(a[q][2 * m + 1], vv.y, fma(a[q][2 * m], vv.x, s[q]));
       }
-      double sp = s0 + s1;
-      sp += __shfl_xor_sync(0xffffffffu, sp, 1);
-      double pv = 0.0;
-      if (i < m && (tid & 1) == 0) {
-        const double p = b * sp;
-        pw[i]          = p;
-        pv             = p * v[i];
-      }
-      pv = warp_sum(pv);
-      if (lane == 0)
-        red[warp] = pv;
-    }
+    // sums over the half-warp: lanes with bit 3 keep rows 2, 3, then bit 2 picks one of the two
+    const bool   b3 = lane & 8, b2 = lane & 4;
+    const double u0 = (b3 ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, b3 ? s[0] : s[2], 8);
+    const double u1 = (b3 ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, b3 ? s[1] : s[3], 8);
+    double       pi = (b2 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b2 ? u0 : u1, 4);
+    pi += __shfl_xor_sync(0xffffffffu, pi, 2);
+    pi += __shfl_xor_sync(0xffffffffu, pi, 1);
+    pi = ip > k ? b * pi : 0.0; // the finished rows take no update
+    if ((lane & 3) == 0)
+      pw[ip] = pi;
+    double pv = pi * vi; // the warp's eight rows
+    pv += __shfl_xor_sync(0xffffffffu, pv, 4);
+    pv += __shfl_xor_sync(0xffffffffu, pv, 8);
+    pv += __shfl_xor_sync(0xffffffffu, pv, 16);
+    if (lane == 0)
+      red[warp] = pv;
     __syncthreads();
-    double dot = 0.0; // p^T v, summed in warp order
+    // A' = A - v p^T - p v^T + kk v v^T with kk = beta p^T v, that is A - v p^T - (p - kk v) v^T
+    if (live) {
+      double dp[kWarps];
 #pragma unroll
-    for (int q = 0; q < kEigWarps; ++q)
-      dot += red[q];
-    const double kk = 0.5 * b * dot; // w = p - kk v
-    if (warp == 0) {
-      // the trailing block's column 0 (column k+1 of A), then the house vector of step k+1 from it
-      const double w0 = fma(-kk, v[0], pw[0]), v0 = v[0];
-      for (int i = lane; i < m; i += 32) {
-        const double wi = fma(-kk, v[i], pw[i]);
-        double      &a  = A[(k + 1 + i) * ld + k + 1];
-        a               = fma(-v[i], w0, fma(-wi, v0, a));
-      }
-      __syncwarp();
-      if (k + 3 < n)
-        house(k + 1);
-    } else { // columns 1 .. m-1, a row at a time per warp; lane owns columns 1 + lane + 32 c
-      double vj[kEigMaxN / 32], wj[kEigMaxN / 32];
+      for (int q = 0; q < kWarps; ++q)
+        dp[q] = red[q];
 #pragma unroll
-      for (int c = 0; c < kEigMaxN / 32; ++c) {
-        const int j = 1 + lane + 32 * c;
-        vj[c]       = j < m ? v[j] : 0.0;
-        wj[c]       = j < m ? fma(-kk, v[j], pw[j]) : 0.0;
-      }
-      for (int i = warp - 1; i < m; i += kEigWarps - 1) {
-        const double vi = v[i], wi = fma(-kk, v[i], pw[i]);
-        double      *row = A + (k + 1 + i) * ld + k + 1;
+      for (int h = kWarps / 2; h > 0; h >>= 1)
 #pragma unroll
-        for (int c = 0; c < kEigMaxN / 32; ++c) {
-          const int j = 1 + lane + 32 * c;
-          if (j < m)
-            row[j] = fma(-vi, wj[c], fma(-wi, vj[c], row[j]));
+        for (int q = 0; q < h; ++q)
+          dp[q] += dp[q + h];
+      const double  kk = b * dp[0];
+      const double2 va = *reinterpret_cast<const double2 *>(v + i0), vb = *reinterpret_cast<const double2 *>(v + i0 + 2);
+      const double2 pa = *reinterpret_cast<const double2 *>(pw + i0), pb = *reinterpret_cast<const double2 *>(pw + i0 + 2);
+      const double  vr[4] = {va.x, va.y, vb.x, vb.y};
+      const double  pk[4] = {fma(-kk, va.x, pa.x), fma(-kk, va.y, pa.y), fma(-kk, vb.x, pb.x), fma(-kk, vb.y, pb.y)};
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        if (32 * m + 31 > k) {
+          const double2 vv = *reinterpret_cast<const double2 *>(v + 2 * tc + 32 * m);
+          const double2 pp = *reinterpret_cast<const double2 *>(pw + 2 * tc + 32 * m);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            a[q][2 * m]     = fma(-pk[q], vv.x, fma(-vr[q], pp.x, a[q][2 * m]));
+            a[q][2 * m + 1] = fma(-pk[q], vv.y, fma(-vr[q], pp.y, a[q][2 * m + 1]));
+          }
         }
-      }
+      if (i0 == ((k + 1) & ~3) && k + 3 < n)
+        house(k + 1);
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    for (int k = n - 2; k < n; ++k)
-      if (k >= 0)
-        d[k] = A[k * ld + k];
-    if (n >= 2)
-      e[n - 2] = A[(n - 1) * ld + n - 2];
-    if (n >= 1)
-      e[n - 1] = 0.0;
-  }
+  // the last two rows
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int c = 0; c < 2 * M; ++c) {
+      const int i = i0 + q, j = 2 * tc + (c & 1) + 32 * (c >> 1);
+      if (i < n && i >= n - 2 && j == i)
+        d[i] = a[q][c];
+      if (i < n && i >= n - 2 && j == i + 1 && j < n)
+        e[i] = a[q][c];
+    }
+  if (tid == 0)
+    e[n - 1] = 0.0;
   __syncthreads();
-  // Gershgorin bounds and ||T|| (warp 0)
+    // Gershgorin bounds and ||T|| (warp 0)
   if (warp == 0) {
     double lo = DBL_MAX, hi = -DBL_MAX, nrm = 0.0;
     for (int i = lane; i < n; i += 32) {
@@ -265,29 +350,30 @@ __global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, do
   }
   __syncthreads();
   const double sc = red[3];
-  for (int i = tid; i < n; i += kEigThr) { // the Sturm sequences run on T sc (exactly scaled)
-    const double es = e[i] * sc;
-    ds[i]           = d[i] * sc;
-    e2[i]           = es * es;
+  // the Sturm sequences run on T sc (exactly scaled), padded to whole groups of four by steps that
+  // change no sign
+  for (int i = tid; i < n + 8; i += NT) {
+    const double es = i + 1 < n ? e[i] * sc : 0.0;
+    ds[i]           = i < n ? d[i] * sc : 2.0;
+    e2[i]           = i + 1 < n ? fmax(es * es, 0x1p-120) : 0.0;
   }
   __syncthreads();
 
-  // ---- 2. eigenvalues n-1, n-2, ..., n-r by multisection, a warp each: 32 shifts per round ------
-  for (int t = warp; t < r; t += kEigWarps) {
+  // ---- 2. eigenvalues n-1, n-2, ..., n-r by multisection, a warp each: 32 shifts per round, until
+  //         the bracket is below the rounding of ||T|| ---------------------------------------------
+  for (int t = warp; t < r; t += kWarps) {
     const int idx = n - 1 - t; // ascending index: count(a) <= idx < count(b)
     double    a = red[0] * sc, b = red[1] * sc;
     for (int round = 0; round < 24; ++round) {
-      const double x   = a + (b - a) * (double)(lane + 1) / 33.0;
-      const int    c   = sturm_count(ds, e2, n, x);
+      const double   w = (b - a) * (1.0 / 33.0);
+      const int      c = sturm_count(ds, e2, n, fma(w, (double)(lane + 1), a));
       const unsigned m = __ballot_sync(0xffffffffu, c > idx);
-      const int    f   = m ? __ffs(m) - 1 : 32; // first shift with more than idx eigenvalues below
-      const double xf  = __shfl_sync(0xffffffffu, x, f & 31);
-      const double xp  = __shfl_sync(0xffffffffu, x, (f + 31) & 31);
-      const double na  = f == 0 ? a : xp;
-      const double nb  = f == 32 ? b : xf;
-      a                = na;
-      b                = nb;
-      if (b - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)) + DBL_MIN)
+      const int      f = m ? __ffs(m) - 1 : 32; // the first shift with more than idx eigenvalues below
+      const double   na = f == 0 ? a : fma(w, (double)f, a);
+      const double   nb = f == 32 ? b : fma(w, (double)(f + 1), a);
+      a                 = na;
+      b                 = nb;
+      if (b - a <= fmax(2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)), 0x1p-54))
         break;
     }
     if (lane == 0)
@@ -295,17 +381,17 @@ __global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, do
   }
   __syncthreads();
 
-  // ---- 3. eigenvectors of T by inverse iteration: eigenvalue t in warp t % 8, whose lane 0 runs
+  // ---- 3. eigenvectors of T by inverse iteration: eigenvalue t in warp t % kWarps, whose lane 0 runs
   //         the LU factorisation and the solves while the warp normalises; close eigenvalues are
   //         orthogonalised in descending order between block barriers ----------------------------
   {
     const double  nrm  = red[2];
     const double  tiny = DBL_EPSILON * nrm + DBL_MIN; // pivot floor
-    const double  clus = 1e-7 * nrm;                  // eigenvalues closer than this share a cluster
-    constexpr int kPer = kEigMaxR / kEigWarps;         // eigenvalues per warp
+    const double  clus = 1e-7 * nrm + 8.0 * DBL_MIN;  // eigenvalues closer than this share a cluster
+    constexpr int kPer = (kEigMaxR + kWarps - 1) / kWarps; // eigenvalues per warp
     uint32_t      swp[kPer][kEigMaxN / 32];            // row j and j+1 exchanged at step j
     for (int u = 0; u < kPer; ++u) {
-      const int t = warp + kEigWarps * u;
+      const int t = warp + kWarps * u;
 #pragma unroll
       for (int q = 0; q < kEigMaxN / 32; ++q)
         swp[u][q] = 0u;
@@ -322,59 +408,81 @@ __global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, do
         double       a0 = d[0] - lm, a1 = n > 1 ? e[0] : 0.0;
         for (int j = 0; j + 1 < n; ++j) {
           const double b0 = e[j], b1 = d[j + 1] - lm, b2 = j + 2 < n ? e[j + 1] : 0.0;
-          if (fabs(a0) >= fabs(b0)) {
-            const double piv = fabs(a0) < tiny ? copysign(tiny, a0) : a0;
-            const double l   = b0 / piv;
-            u0[j] = piv, u1[j] = a1, u2[j] = 0.0, ml[j] = l;
-            a0 = b1 - l * a1;
-            a1 = b2;
-          } else {
-            const double l = a0 / b0;
-            u0[j] = b0, u1[j] = b1, u2[j] = b2, ml[j] = l;
+          const bool   keep = fabs(a0) >= fabs(b0);
+          const double piv  = keep ? (fabs(a0) < tiny ? copysign(tiny, a0) : a0) : b0;
+          const double l    = (keep ? b0 : a0) * reciprocal(piv);
+          u0[j] = piv, ml[j] = l;
+          u1[j] = keep ? a1 : b1, u2[j] = keep ? 0.0 : b2;
+          if (!keep)
             swp[u][j >> 5] |= 1u << (j & 31);
-            a0 = a1 - l * b1;
-            a1 = -l * b2;
-          }
+          a0 = keep ? fma(-l, a1, b1) : fma(-l, b1, a1);
+          a1 = keep ? b2 : -l * b2;
         }
         u0[n - 1] = fabs(a0) < tiny ? copysign(tiny, a0) : a0;
       }
       __syncwarp();
-      for (int j = lane; j < n; j += 32) { // the solves multiply by the pivots' reciprocals
-        u0[j] = 1.0 / u0[j];
+      for (int j = lane; j < n; j += 32) { // U's rows over their pivots: one fused step per entry
+        const double ip = reciprocal(u0[j]);
+        u0[j] = ip;
+        u1[j] = j + 1 < n ? u1[j] * ip : 0.0;
+        u2[j] = j + 2 < n ? u2[j] * ip : 0.0;
         y[j]  = 1.0 + 0.01 * (double)(((j * 7 + t * 13) % 17) - 8); // start: nonzero, distinct per t
       }
     }
     bool clustered = false; // any two of the r eigenvalues closer than clus
     for (int q = 1; q < r; ++q)
       clustered |= fabs(lam[q] - lam[q - 1]) <= clus;
-    for (int it = 0; it < 3; ++it) {
+    for (int it = 0; it < 2; ++it) {
       for (int u = 0; u < kPer; ++u) {
-        const int t = warp + kEigWarps * u;
+        const int t = warp + kWarps * u;
         if (t >= r)
           continue;
         double       *y  = Y + t * ldy;
         const double *u0 = lu + (0 * kEigMaxR + t) * ldy, *u1 = lu + (1 * kEigMaxR + t) * ldy,
                      *u2 = lu + (2 * kEigMaxR + t) * ldy, *ml = lu + (3 * kEigMaxR + t) * ldy;
         __syncwarp();
-        if (lane == 0) { // solve M y' = y in place, the running entry carried in a register
-          double c = y[0];
-          for (int j = 0; j + 1 < n; ++j) {
-            const double nx = y[j + 1];
-            if ((swp[u][j >> 5] >> (j & 31)) & 1u) { // rows j, j+1 exchanged
-              y[j] = nx;
-              c    = c - ml[j] * nx;
-            } else {
-              y[j] = c;
-              c    = nx - ml[j] * c;
-            }
+        if (lane == 0) { // solve M y' = y in place, the running entry carried in a register; eight
+                         // entries are loaded ahead of the chain and stored behind it
+          constexpr int kCh = 8;
+          double        c   = y[0];
+          for (int j0 = 0; j0 + 1 < n; j0 += kCh) {
+            double nx[kCh], l[kCh], o[kCh];
+#pragma unroll
+            for (int i = 0; i < kCh; ++i)
+              if (j0 + i + 1 < n)
+                nx[i] = y[j0 + i + 1], l[i] = ml[j0 + i];
+            const uint32_t sw = swp[u][j0 >> 5] >> (j0 & 31);
+#pragma unroll
+            for (int i = 0; i < kCh; ++i)
+              if (j0 + i + 1 < n) {
+                const bool ex2 = (sw >> i) & 1u; // rows j, j+1 exchanged
+                o[i] = ex2 ? nx[i] : c;
+                c    = ex2 ? fma(-l[i], nx[i], c) : fma(-l[i], c, nx[i]);
+              }
+#pragma unroll
+            for (int i = 0; i < kCh; ++i)
+              if (j0 + i + 1 < n)
+                y[j0 + i] = o[i];
           }
           double c1 = c * u0[n - 1], c2 = 0.0; // y[j+1], y[j+2] of the back substitution
           y[n - 1]  = c1;
-          for (int j = n - 2; j >= 0; --j) {
-            const double c0 = (y[j] - u1[j] * c1 - u2[j] * c2) * u0[j];
-            y[j]            = c0;
-            c2              = c1;
-            c1              = c0;
+          for (int j0 = n - 2; j0 >= 0; j0 -= kCh) {
+            double yy[kCh], a1[kCh], a2[kCh];
+#pragma unroll
+            for (int i = 0; i < kCh; ++i)
+              if (j0 - i >= 0)
+                yy[i] = y[j0 - i] * u0[j0 - i], a1[i] = u1[j0 - i], a2[i] = u2[j0 - i];
+#pragma unroll
+            for (int i = 0; i < kCh; ++i)
+              if (j0 - i >= 0) {
+                yy[i] = fma(-a1[i], c1, fma(-a2[i], c2, yy[i]));
+                c2    = c1;
+                c1    = yy[i];
+              }
+#pragma unroll
+            for (int i = 0; i < kCh; ++i)
+              if (j0 - i >= 0)
+                y[j0 - i] = yy[i];
           }
         }
         __syncwarp();
@@ -404,7 +512,7 @@ __global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, do
       __syncthreads();
       // modified Gram-Schmidt within clusters, in descending eigenvalue order, by the warp of s2
       for (int s2 = 1; s2 < r; ++s2) {
-        if (warp == s2 % kEigWarps) {
+        if (warp == s2 % kWarps) {
           double *y   = Y + s2 * ldy;
           bool    any = false;
           for (int q = 0; q < s2; ++q) {
@@ -438,41 +546,89 @@ __global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, do
   }
   __syncthreads();
 
-  // ---- 4. back-transformation V = Q Y, a warp per column, entries i = lane + 32 c in registers ---
-  for (int t = warp; t < r; t += kEigWarps) {
-    const double *ys = Y + t * ldy;
-    double        y[kEigMaxN / 32];
+  // ---- 4. back-transformation V = Q Y by the reflectors in descending order, four at a time: the
+  //         dot products of a block with y run side by side, and the products of its reflectors with
+  //         each other (in G) carry the sequential order.  A warp per column, entries lane + 32 c -----
+  double *G = lu; // [blocks][6]: v_k . v_(k-1), v_k . v_(k-2), v_(k-1) . v_(k-2), then those with v_(k-3)
+  const auto reflector = [&](int k, double (&v)[NC]) { // 0 before k = 0
 #pragma unroll
-    for (int c = 0; c < kEigMaxN / 32; ++c) {
+    for (int c = 0; c < NC; ++c)
+      v[c] = k >= 0 ? R[k * RM + lane + 32 * c] : 0.0;
+  };
+  const int nblk = (max(n - 2, 0) + 3) / 4;
+  for (int bl = warp; bl < nblk; bl += kWarps) {
+    const int k = n - 3 - 4 * bl;
+    double    v[4][NC], g[6];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      reflector(k - q, v[q]);
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+#pragma unroll
+      for (int h = 0; h < q; ++h) {
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          s = fma(v[q][c], v[h][c], s);
+        g[q * (q - 1) / 2 + h] = warp_sum(s);
+      }
+    if (lane < 6) {
+      double x = g[0];
+#pragma unroll
+      for (int q = 1; q < 6; ++q)
+        x = lane == q ? g[q] : x;
+      G[6 * bl + lane] = x;
+    }
+  }
+  __syncthreads();
+  for (int t = warp; t < r; t += kWarps) {
+    const double *ys = Y + t * ldy;
+    double        y[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
       const int i = lane + 32 * c;
       y[c]        = i < n ? ys[i] : 0.0;
     }
-    for (int k = n - 3; k >= 0; --k) {
-      const double b = beta[k];
-      if (b == 0.0)
-        continue;
-      double vr[kEigMaxN / 32], s = 0.0; // reflector k: column k of A, rows k+1 .. n-1
+    for (int bl = 0; bl < nblk; ++bl) {
+      const int k = n - 3 - 4 * bl;
+      double    v[4][NC], s[4], cf[4];
 #pragma unroll
-      for (int c = 0; c < kEigMaxN / 32; ++c) {
-        const int i = lane + 32 * c;
-        vr[c]       = i > k && i < n ? A[i * ld + k] : 0.0;
-        s           = fma(vr[c], y[c], s);
+      for (int q = 0; q < 4; ++q) {
+        reflector(k - q, v[q]);
+        s[q] = 0.0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          s[q] = fma(v[q][c], y[c], s[q]);
       }
-      s = b * warp_sum(s);
 #pragma unroll
-      for (int c = 0; c < kEigMaxN / 32; ++c)
-        y[c] = fma(-s, vr[c], y[c]);
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { // coefficient of reflector k - q after the ones before it
+        double x = s[q];
+#pragma unroll
+        for (int h = 0; h < q; ++h)
+          x = fma(-cf[h], G[6 * bl + q * (q - 1) / 2 + h], x);
+        cf[q] = k - q >= 0 ? beta[k - q] * x : 0.0;
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          y[c] = fma(-cf[q], v[q][c], y[c]);
     }
     const int idx = n - 1 - t;
     double   *vec = evecs + (int64_t)blockIdx.x * n * n;
 #pragma unroll
-    for (int c = 0; c < kEigMaxN / 32; ++c) {
+    for (int c = 0; c < NC; ++c) {
       const int i = lane + 32 * c;
       if (i < n)
         vec[i * n + idx] = y[c];
     }
     if (lane == 0)
-      evals[(int64_t)blockIdx.x * n + idx] = lam[t];
+      evals[(int64_t)blockIdx.x * n + idx] = ldexp(lam[t], ex);
   }
   if (tid == 0 && info != nullptr)
     info[blockIdx.x] = 0;
@@ -481,9 +637,8 @@ __global__ void __launch_bounds__(kEigThr) eig_top_kernel(const double *a_in, do
 } // namespace
 
 size_t eig_top_smem_bytes(int n) {
-  return ((size_t)n * (n + 1) + 8 * (size_t)n + kEigMaxR + 5 * (size_t)kEigMaxR * eig_ldy(n) + kEigWarps + 4) *
-             sizeof(double) +
-         16;
+  return ((size_t)(n + 1) * (eig_threads(n) / 4) + 5 * (size_t)n + 16 + kEigMaxR + 5 * (size_t)kEigMaxR * eig_ldy(n) +
+          kEigRed) * sizeof(double) + 16;
 }
 
 bool eig_top_supported(int n, int r) { return n >= 1 && n <= kEigMaxN && r >= 1 && r <= kEigMaxR && r <= n; }
@@ -492,8 +647,10 @@ int launch_eig_top(const double *a, double *evecs, double *evals, int *info, int
                    cudaStream_t s) {
   HF_CHECK_ARG(eig_top_supported(n, r) && batch >= 1, "eig_top: order must be in [1, 128] and 1 <= r <= min(16, n)");
   const size_t smem = eig_top_smem_bytes(n);
-  HF_CUDA(cudaFuncSetAttribute(eig_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  eig_top_kernel<<<(unsigned)batch, kEigThr, smem, s>>>(a, evecs, evals, info, n, r);
+  const int    nt   = eig_threads(n);
+  auto         kern = nt == 128 ? eig_top_kernel<128> : (nt == 256 ? eig_top_kernel<256> : eig_top_kernel<512>);
+  HF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<(unsigned)batch, nt, smem, s>>>(a, evecs, evals, info, n, r);
   note_launch();
   return launch_status("eig_top_kernel");
 }

