@@ -3,9 +3,8 @@
 //
 // Reference: PcaTask::execute (holotask/src/syncs/pca.cc:68-119) computes C = X^T X with
 // cublasGemmEx (FP16 tensor-core compute), an ascending eigendecomposition with cuSolverDx heev
-// (pca_heev.cc:35-133) and the projection X V[:, begin:end].  Here the Gram matrix is
-// accumulated in FP32 over pixel tiles on shifted samples (x - 2048 is exact for 12-bit data)
-// and reduced in FP64 with the shift undone exactly; the eigensolver is FP64 throughout.
+// (pca_heev.cc:35-133) and the projection X V[:, begin:end].  Here the Gram matrix comes from
+// k_cov_fp32.cu or k_tc_cov.cu; the eigensolver is FP64 throughout.
 #include <algorithm>
 #include <cfloat>
 #include <mutex>
@@ -17,165 +16,8 @@ namespace hf {
 
 namespace {
 
-constexpr int kCovPT = 128; // pixels per tile
-
-template <int T> struct CovGeom {
-  static constexpr int NB     = T / 4;                 // 4x4 blocks per side
-  static constexpr int U      = NB * (NB + 1) / 2;     // upper-triangle blocks
-  static constexpr int G      = T == 32 ? 4 : (T == 64 ? 2 : 1); // pixel groups
-  static constexpr int THR    = U * G;
-  static constexpr int XS     = T + 4;                 // padded row of the unpacked tile
-};
-
-template <int FMT> struct Bpp;  // bytes per pixel (numerator / denominator)
-template <> struct Bpp<HF_MONO12P> { static constexpr int num = 3, den = 2; };
-template <> struct Bpp<HF_U16> { static constexpr int num = 2, den = 1; };
-template <> struct Bpp<HF_U8> { static constexpr int num = 1, den = 1; };
-template <> struct Bpp<HF_F32> { static constexpr int num = 4, den = 1; };
-
-template <int FMT, int T>
-__global__ void __launch_bounds__(CovGeom<T>::THR) cov_tiled_kernel(CovArgs a) {
-  using Gm = CovGeom<T>;
-  constexpr int RB  = kCovPT * Bpp<FMT>::num / Bpp<FMT>::den; // packed bytes per frame row
-  constexpr int RW  = RB / 4 + 1;                             // padded words per staged row
-  extern __shared__ __align__(16) uint8_t smem[];
-  uint32_t *stage = reinterpret_cast<uint32_t *>(smem);             // [T][RW]
-  float    *xs    = reinterpret_cast<float *>(smem + T * RW * 4);  // [PT][XS]
-  unsigned long long *ssum = reinterpret_cast<unsigned long long *>(xs + kCovPT * Gm::XS); // [T]
-
-  const int tid = threadIdx.x;
-  const int w   = blockIdx.y;
-  const int grp = tid / Gm::U, blk = tid % Gm::U;
-  // upper-triangle block index -> (bi, bj), bi <= bj
-  int bi = 0, rem = blk;
-  while (rem >= Gm::NB - bi) {
-    rem -= Gm::NB - bi;
-    ++bi;
-  }
-  const int bj = bi + rem;
-
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      acc[i][j] = 0.f;
-  for (int t = tid; t < T; t += blockDim.x)
-    ssum[t] = 0;
-
-  const int64_t ntiles = (a.P + kCovPT - 1) / kCovPT;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t p0 = tile * kCovPT;
-    const int     np = (int)min((int64_t)kCovPT, a.P - p0);
-    const int     nw = (np * Bpp<FMT>::num / Bpp<FMT>::den + 3) / 4;
-    __syncthreads();
-    for (int i = tid; i < T * (RB / 4); i += blockDim.x) {
-      const int t = i / (RB / 4), j = i % (RB / 4);
-      const uint32_t *src = reinterpret_cast<const uint32_t *>(
-          a.ring.frame(w, t) + p0 * Bpp<FMT>::num / Bpp<FMT>::den);
-      stage[t * RW + j] = j < nw ? __ldg(src + j) : 0u;
-    }
-    __syncthreads();
-    // unpack: thread (t, 8-pixel group); lanes run along t (conflict-free xs writes)
-    for (int i = tid; i < T * (kCovPT / 8); i += blockDim.x) {
-      const int t = i % T, g = i / T;
-      float     v[8];
-      if constexpr (FMT == HF_MONO12P) {
-        uint32_t p[8];
-        unpack8(stage[t * RW + 3 * g], stage[t * RW + 3 * g + 1], stage[t * RW + 3 * g + 2], p);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          v[k] = (float)p[k];
-      } else if constexpr (FMT == HF_U16) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t wv = stage[t * RW + 4 * g + k];
-          v[2 * k]     = (float)(wv & 0xFFFFu);
-          v[2 * k + 1] = (float)(wv >> 16);
-        }
-      } else if constexpr (FMT == HF_U8) {
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const uint32_t wv = stage[t * RW + 2 * g + k];
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            v[4 * k + j] = (float)((wv >> (8 * j)) & 0xFFu);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          v[k] = __uint_as_float(stage[t * RW + 8 * g + k]);
-      }
-      unsigned int isum = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int p = 8 * g + k;
-        const bool in = p < np;
-        if constexpr (FMT != HF_F32)
-          isum += in ? (unsigned int)v[k] : 0u;
-        xs[p * Gm::XS + t] = in ? v[k] - a.shift : 0.f;
-      }
-      if constexpr (FMT != HF_F32)
-        atomicAdd(&ssum[t], (unsigned long long)isum);
-    }
-    __syncthreads();
-    // accumulate this group's share of the tile
-    if (grp < Gm::G) {
-      for (int p = grp; p < kCovPT; p += Gm::G) {
-        const float4 xa = *reinterpret_cast<const float4 *>(xs + p * Gm::XS + 4 * bi);
-        const float4 xb = *reinterpret_cast<const float4 *>(xs + p * Gm::XS + 4 * bj);
-        const float  va[4] = {xa.x, xa.y, xa.z, xa.w};
-        const float  vb[4] = {xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            acc[i][j] = fmaf(va[i], vb[j], acc[i][j]);
-      }
-    }
-  }
-  __syncthreads();
-  if (grp < Gm::G) {
-    const int64_t pidx = ((int64_t)w * a.nblk + (int64_t)blockIdx.x * Gm::G + grp) * T * T;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        a.partial[pidx + (4 * bi + i) * T + 4 * bj + j] = acc[i][j];
-  }
-  for (int t = tid; t < T; t += blockDim.x)
-    a.sums[((int64_t)w * gridDim.x + blockIdx.x) * T + t] = (double)ssum[t];
-}
-
-// Deterministic reduction of the partials; undoes the shift exactly (float64).
-__global__ void cov_finalize_kernel(const float *partial, const double *sums, int nblk,
-                                    int nsum, int T, int64_t P, double shift, double *gram) {
-  const int w = blockIdx.y;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= T * T)
-    return;
-  const int i = e / T, j = e % T;
-  if (i > j)
-    return;
-  // the tiled kernel writes every entry (i, j) with block(i) <= block(j), so i <= j is present
-  double g = 0.0;
-  const float *pp = partial + (int64_t)w * nblk * T * T + i * T + j;
-  for (int b = 0; b < nblk; ++b)
-    g += (double)pp[(int64_t)b * T * T];
-  if (shift != 0.0) {
-    double si = 0.0, sj = 0.0;
-    const double *sp = sums + (int64_t)w * nsum * T;
-    for (int b = 0; b < nsum; ++b) {
-      si += sp[(int64_t)b * T + i];
-      sj += sp[(int64_t)b * T + j];
-    }
-    g += shift * (si + sj) - shift * shift * (double)P;
-  }
-  gram[(int64_t)w * T * T + i * T + j] = g;
-  gram[(int64_t)w * T * T + j * T + i] = g;
-}
-
-// Any T (small problems): one thread per upper entry, float64 accumulation, no shift.
+// Any T, no workspace (more than 128 frames, or callers without one): one thread per upper entry,
+// float64 accumulation, no shift.
 template <int FMT>
 __global__ void cov_generic_kernel(FrameRing ring, int T, int64_t P, double *gram) {
   const int w = blockIdx.y;
@@ -193,56 +35,21 @@ __global__ void cov_generic_kernel(FrameRing ring, int T, int64_t P, double *gra
   gram[(int64_t)w * T * T + j * T + i] = g;
 }
 
-int cov_ctas_per_window(int64_t P, int nwin) {
-  const int64_t ntiles = (P + kCovPT - 1) / kCovPT;
-  int           ctas   = (2 * sm_count() + nwin - 1) / nwin;
-  ctas = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, ntiles));
-  return ctas;
-}
-
-// `max_ctas` > 0 caps the CTAs per window (and so the workspace) below the default split.
-template <int FMT, int T>
-int launch_cov_tiled(const FrameRing &ring, int64_t P, int nwin, void *ws, double *gram,
-                     cudaStream_t s, int max_ctas = 0) {
-  using Gm = CovGeom<T>;
-  constexpr int RB   = kCovPT * Bpp<FMT>::num / Bpp<FMT>::den;
-  constexpr int RW   = RB / 4 + 1;
-  const size_t  smem = (size_t)T * RW * 4 + (size_t)kCovPT * Gm::XS * 4 + T * 8;
-  const int     ctas = max_ctas > 0 ? std::min(max_ctas, cov_ctas_per_window(P, nwin))
-                                    : cov_ctas_per_window(P, nwin);
-  CovArgs       a;
-  a.ring    = ring;
-  a.T       = T;
-  a.P       = P;
-  a.shift   = FMT == HF_F32 ? 0.f : (FMT == HF_U8 ? 128.f : 2048.f);
-  a.nblk    = ctas * Gm::G;
-  a.partial = reinterpret_cast<float *>(ws);
-  a.sums    = reinterpret_cast<double *>(reinterpret_cast<uint8_t *>(ws) +
-                                      (size_t)nwin * a.nblk * T * T * sizeof(float));
-  HF_CUDA(cudaFuncSetAttribute(cov_tiled_kernel<FMT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
-  cov_tiled_kernel<FMT, T><<<dim3(ctas, nwin), Gm::THR, smem, s>>>(a);
-  note_launch();
-  HF_TRY(launch_status("cov_tiled_kernel"));
-  return launch_cov_finalize(a.partial, a.sums, a.nblk, ctas, T, P, (double)a.shift, gram, nwin, s);
-}
-
 template <int FMT>
-int launch_cov_fmt(const FrameRing &ring, int T, int64_t P, int nwin, void *ws, double *gram,
-                   cudaStream_t s) {
-  if constexpr (FMT != HF_CF32) {
-    // the tiled kernel reads frames as 4-byte words: the base must be 4-byte aligned too
-    const bool tiled = (P % 8 == 0) && (ring.frame_bytes % 4 == 0) && (((uintptr_t)ring.base & 3) == 0);
-    if (tiled && T == 32)
-      return launch_cov_tiled<FMT, 32>(ring, P, nwin, ws, gram, s);
-    if (tiled && T == 64)
-      return launch_cov_tiled<FMT, 64>(ring, P, nwin, ws, gram, s);
-    if (tiled && T == 128)
-      return launch_cov_tiled<FMT, 128>(ring, P, nwin, ws, gram, s);
-  }
+int launch_cov_generic(const FrameRing &ring, int T, int64_t P, int nwin, double *gram, cudaStream_t s) {
   cov_generic_kernel<FMT><<<dim3((T * T + 127) / 128, nwin), 128, 0, s>>>(ring, T, P, gram);
   note_launch();
   return launch_status("cov_generic_kernel");
+}
+
+int launch_cov_direct(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, double *gram, cudaStream_t s) {
+  switch (fmt) {
+  case HF_MONO12P: return launch_cov_generic<HF_MONO12P>(ring, T, P, nwin, gram, s);
+  case HF_U16: return launch_cov_generic<HF_U16>(ring, T, P, nwin, gram, s);
+  case HF_U8: return launch_cov_generic<HF_U8>(ring, T, P, nwin, gram, s);
+  case HF_F32: return launch_cov_generic<HF_F32>(ring, T, P, nwin, gram, s);
+  default: return fail(HF_ERR_INVALID, "covariance: unsupported input dtype");
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -548,30 +355,16 @@ __global__ void pca_project_kernel(const float *in, int T, int64_t P, const doub
 
 } // namespace
 
-int launch_cov_finalize(const float *partial, const double *sums, int nblk, int nsum, int T, int64_t P,
-                        double shift, double *gram, int nwin, cudaStream_t s) {
-  cov_finalize_kernel<<<dim3((T * T + 255) / 256, nwin), 256, 0, s>>>(partial, sums, nblk, nsum, T, P, shift,
-                                                                      gram);
-  note_launch();
-  return launch_status("cov_finalize_kernel");
-}
-
 size_t cov_workspace_bytes(int T, int64_t P, int nwin) {
-  const int ctas = cov_ctas_per_window(P, nwin);
-  const int G    = T == 32 ? 4 : (T == 64 ? 2 : 1);
-  return (size_t)nwin * ctas * G * T * T * sizeof(float) + (size_t)nwin * ctas * T * sizeof(double) + 256;
+  return cov_fp32_supported(T) ? cov_fp32_workspace_bytes(T, P, nwin) : 256;
 }
 
 int launch_covariance(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws,
                       double *gram, cudaStream_t s) {
   HF_CHECK_ARG(T > 0 && P > 0 && nwin > 0, "covariance: empty problem");
-  switch (fmt) {
-  case HF_MONO12P: return launch_cov_fmt<HF_MONO12P>(ring, T, P, nwin, ws, gram, s);
-  case HF_U16: return launch_cov_fmt<HF_U16>(ring, T, P, nwin, ws, gram, s);
-  case HF_U8: return launch_cov_fmt<HF_U8>(ring, T, P, nwin, ws, gram, s);
-  case HF_F32: return launch_cov_fmt<HF_F32>(ring, T, P, nwin, ws, gram, s);
-  default: return fail(HF_ERR_INVALID, "covariance: unsupported input dtype");
-  }
+  if (ws != nullptr && cov_fp32_supported(T))
+    return launch_cov_fp32(ring, fmt, T, P, nwin, ws, gram, 0, s);
+  return launch_cov_direct(ring, fmt, T, P, nwin, gram, s);
 }
 
 int launch_jacobi(const double *a, double *evecs, double *evals, int *info, int n, int64_t batch,
@@ -620,7 +413,7 @@ int launch_pca_project(const float *in, int64_t batch, int T, int64_t P, const d
 //
 // The workspace is a file-scope device array, so the module loader reserves it once per device
 // and the call itself never allocates.  Its device address is looked up once per device (with
-// that device current) and cached.  The tiled kernel writes every partial and per-frame sum the
+// that device current) and cached.  The kernel writes every partial and per-frame sum the
 // reduction reads before it is read, so nothing in the array has to start at zero.  Every call
 // on a device uses the same array: calls whose work overlaps in time race on it.
 // ------------------------------------------------------------------------------------------------
@@ -647,56 +440,34 @@ int scratch_address(void **ptr) {
   return HF_OK;
 }
 
-// CTAs per window that fit the fixed workspace (0 when even one does not).
-template <int T> int fitting_ctas(int nwin) {
-  using Gm                 = CovGeom<T>;
-  const size_t per_cta     = (size_t)Gm::G * T * T * sizeof(float) + (size_t)T * sizeof(double);
-  const size_t usable      = HF_COVARIANCE_NOALLOC_SCRATCH_BYTES - 256;
-  const size_t fit         = usable / ((size_t)nwin * per_cta);
-  return (int)std::min<size_t>(fit, (size_t)1 << 20);
-}
-
-template <int FMT, int T>
-int cov_fixed_tiled(const FrameRing &ring, int64_t P, int nwin, void *ws, double *gram, cudaStream_t s) {
-  const int fit = fitting_ctas<T>(nwin);
-  if (fit < 1)
-    return fail(HF_ERR_INVALID,
-                "hf_covariance_noalloc: batch " + std::to_string(nwin) + " at T = " + std::to_string(T) +
-                    " needs more than the fixed " +
-                    std::to_string(HF_COVARIANCE_NOALLOC_SCRATCH_BYTES >> 20) +
-                    " MiB workspace; split the batch or use hf_covariance with a workspace");
-  return launch_cov_tiled<FMT, T>(ring, P, nwin, ws, gram, s, fit);
-}
-
-template <int FMT>
-int cov_fixed_fmt(const FrameRing &ring, int T, int64_t P, int nwin, double *gram, cudaStream_t s) {
-  const bool tiled = (P % 8 == 0) && (ring.frame_bytes % 4 == 0) && (((uintptr_t)ring.base & 3) == 0) &&
-                     (T == 32 || T == 64 || T == 128);
-  if (!tiled) { // the direct kernel needs no workspace (and takes any alignment)
-    cov_generic_kernel<FMT><<<dim3((T * T + 127) / 128, nwin), 128, 0, s>>>(ring, T, P, gram);
-    note_launch();
-    return launch_status("cov_generic_kernel");
-  }
-  void *ws = nullptr;
-  HF_TRY(scratch_address(&ws));
-  if (T == 32)
-    return cov_fixed_tiled<FMT, 32>(ring, P, nwin, ws, gram, s);
-  if (T == 64)
-    return cov_fixed_tiled<FMT, 64>(ring, P, nwin, ws, gram, s);
-  return cov_fixed_tiled<FMT, 128>(ring, P, nwin, ws, gram, s);
+// One CTA's partials as the batch limit counts them.  T = 32, 64 and 128 on 4-byte-aligned rows keep
+// the documented T*T*4*G + T*8 bytes (the kernel needs no more); the others, which have no limit, count
+// what the kernel writes and take the direct kernel beyond it.
+size_t fixed_cta_bytes(int T, bool limited) {
+  const int G = T == 32 ? 4 : (T == 64 ? 2 : 1);
+  return limited ? (size_t)G * T * T * sizeof(float) + (size_t)T * sizeof(double) : cov_fp32_cta_bytes(T);
 }
 } // namespace
 
 int launch_covariance_fixed_scratch(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, double *gram,
                                     cudaStream_t s) {
   HF_CHECK_ARG(T > 0 && P > 0 && nwin > 0, "covariance: empty problem");
-  switch (fmt) {
-  case HF_MONO12P: return cov_fixed_fmt<HF_MONO12P>(ring, T, P, nwin, gram, s);
-  case HF_U16: return cov_fixed_fmt<HF_U16>(ring, T, P, nwin, gram, s);
-  case HF_U8: return cov_fixed_fmt<HF_U8>(ring, T, P, nwin, gram, s);
-  case HF_F32: return cov_fixed_fmt<HF_F32>(ring, T, P, nwin, gram, s);
-  default: return fail(HF_ERR_INVALID, "covariance: unsupported input dtype");
+  const bool limited = (T == 32 || T == 64 || T == 128) && P % 8 == 0 && ring.frame_bytes % 4 == 0 &&
+                       (reinterpret_cast<uintptr_t>(ring.base) & 3) == 0;
+  const size_t usable = HF_COVARIANCE_NOALLOC_SCRATCH_BYTES - 256;
+  const size_t fit    = cov_fp32_supported(T) ? usable / ((size_t)nwin * fixed_cta_bytes(T, limited)) : 0;
+  if (fit < 1) {
+    if (!limited)
+      return launch_cov_direct(ring, fmt, T, P, nwin, gram, s);
+    return fail(HF_ERR_INVALID,
+                "hf_covariance_noalloc: batch " + std::to_string(nwin) + " at T = " + std::to_string(T) +
+                    " needs more than the fixed " +
+                    std::to_string(HF_COVARIANCE_NOALLOC_SCRATCH_BYTES >> 20) +
+                    " MiB workspace; split the batch or use hf_covariance with a workspace");
   }
+  void *ws = nullptr;
+  HF_TRY(scratch_address(&ws));
+  return launch_cov_fp32(ring, fmt, T, P, nwin, ws, gram, (int)std::min<size_t>(fit, (size_t)1 << 20), s);
 }
 
 } // namespace hf

@@ -19,6 +19,13 @@ struct CovArgs {
 };
 
 size_t cov_workspace_bytes(int T, int64_t P, int nwin);
+// FP32 CUDA-core Gram matrix, T <= 128, any row alignment (k_cov_fp32.cu); `max_ctas` > 0 caps the CTAs
+// per window, each of which writes cov_fp32_cta_bytes of partials.
+bool   cov_fp32_supported(int T);
+size_t cov_fp32_cta_bytes(int T);
+size_t cov_fp32_workspace_bytes(int T, int64_t P, int nwin);
+int    launch_cov_fp32(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram,
+                       int max_ctas, cudaStream_t s);
 // Deterministic float64 reduction of block partials; undoes the sample shift exactly.
 int launch_cov_finalize(const float *partial, const double *sums, int nblk, int nsum, int T, int64_t P,
                         double shift, double *gram, int nwin, cudaStream_t s);
@@ -31,7 +38,8 @@ bool   cov_tc_supported(int fmt, int T, int64_t P, int64_t frame_bytes);
 size_t cov_tc_workspace_bytes(int T, int64_t P, int nwin);
 int    launch_covariance_tc(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws,
                             double *gram, int *status, cudaStream_t s);
-// Full Gram computation: block partials -> deterministic float64 reduction -> gram[nwin][T][T].
+// Full Gram computation: block partials -> deterministic float64 reduction -> gram[nwin][T][T].  A
+// null `ws`, or T > 128, takes the direct kernel.
 int launch_covariance(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws,
                       double *gram, cudaStream_t s);
 // The same computation on the library's fixed device workspace (no allocation; see

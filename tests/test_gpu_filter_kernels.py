@@ -94,3 +94,37 @@ def test_band_matrix_staged_and_direct(cuda, T, rank, z0, z1):
     for b in range(2):
         exp = O.band_matrix(T, z0, z1, V[b][:, T - rank:])
         assert np.abs(w[b].cpu().numpy() - exp).max() < 2.0 ** -22 * np.abs(exp).max() + 1e-14
+
+
+@pytest.mark.parametrize("fmt", ["u8", "u16", "f32", "mono12p"])
+@pytest.mark.parametrize("T,P", [(1, 64), (7, 30), (8, 257), (16, 4098), (33, 1000), (50, 2050), (64, 4096), (100, 514),
+                                 (128, 3002), (130, 66)])
+def test_fp32_gram_any_length_and_alignment(cuda, fmt, T, P):
+    """Block edges, ragged tiles, rows of any alignment; with and without a workspace."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    if fmt == "mono12p" and P % 2:
+        pytest.skip("packed frames have an even pixel count")
+    rng = np.random.default_rng(T * P)
+    top = {"u8": 256, "u16": 65536, "f32": 4096, "mono12p": 4096}[fmt]
+    x = rng.integers(0, top, (2, T, P))
+    if fmt == "mono12p":
+        raw, dt = O.pack12(x.astype(np.uint16).reshape(-1)), hf.HF_MONO12P
+    else:
+        raw, dt = {"u8": (x.astype(np.uint8).reshape(-1), hf.HF_U8),
+                   "u16": (x.astype(np.uint16).reshape(-1).view(np.uint8), hf.HF_U16),
+                   "f32": (x.astype(np.float32).reshape(-1).view(np.uint8), hf.HF_F32)}[fmt]
+    for off in (0, 4):
+        buf = torch.zeros(raw.size + off, dtype=torch.uint8, device=cuda)
+        buf[off:] = torch.from_numpy(raw.copy()).to(cuda)
+        dev = buf[off:]
+        got = [pl.covariance(dev, dt, 2, T, P).cpu().numpy()]
+        noalloc = torch.empty((2, T, T), dtype=torch.float64, device=cuda)
+        got.append(pl.covariance_noalloc(dev, dt, 2, T, P, noalloc).cpu().numpy())
+        for g in got:
+            for b in range(2):
+                X = x[b].astype(np.float64)
+                exp = X @ X.T
+                assert np.abs(g[b] - exp).max() / np.abs(exp).max() < 2e-7
+                assert np.array_equal(g[b], g[b].T)
