@@ -91,3 +91,27 @@ def test_angular_moments(cuda, H, W, pad, nwin, dtype, shift, mask):
         exp = O.reconstruct_window(x[w * T:(w + 1) * T].astype(np.float64), cfg)
         for i, m in enumerate([m for m in range(3) if mask >> m & 1]):
             assert O.rel_l2(got[w, i], exp[m]) < 1e-4, (w, m)
+
+
+@pytest.mark.parametrize("H,W,nwin", [(64, 64, 1), (64, 256, 3), (128, 64, 2), (128, 1024, 1), (256, 128, 1), (256, 512, 2),
+                                      (512, 64, 1), (512, 768, 1)])
+@pytest.mark.parametrize("nz", [1, 4, 5, 16, 31])
+@pytest.mark.parametrize("shift,mask,form", [(0, 7, 0), (1, 6, 1)])
+def test_short_column_moments(cuda, H, W, nwin, nz, shift, mask, form):
+    """Groups of planes in the column pass: one plane, full groups, a remainder, both CTA sizes."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(H * W + nz)
+    T, z0 = 64, 1
+    x = rng.integers(0, 4096, (T * nwin, H, W)).astype(np.uint16)
+    ring = torch.from_numpy(x.view(np.int16)).to(cuda)
+    p = pl.Pipeline(pl.PipelineConfig(height=H, width=W, frames=T, hop=T, z_begin=z0, z_end=z0 + nz,
+                                      input_dtype=hf.HF_U16, z=0.3, max_batch=nwin, fftshift=shift,
+                                      moment_mask=mask, form=form))
+    got = p.run(ring, T * nwin, 0, nwin).cpu().numpy()
+    cfg = O.PathConfig(H, W, T, T, z0, z0 + nz, z=0.3, fftshift=bool(shift))
+    for w in range(nwin):
+        exp = O.reconstruct_window(x[w * T:(w + 1) * T].astype(np.float64), cfg)
+        for i, m in enumerate([m for m in range(3) if mask >> m & 1]):
+            assert O.rel_l2(got[w, i], exp[m]) < (1e-3 if form else 1e-4), (w, m)
