@@ -15,12 +15,22 @@
 // band DFT leaves them.
 //
 // Warp roles (384 threads, one CTA per SM, persistent over segments taken from a counter):
-//   warps 0-3  : load + unpack the next segment into A, rebuild B per window, and (thread 0)
-//                issue the MMAs once the epilogue has released TMEM;
+//   warps 0-3  : unpack the segment into A, rebuild B per window, and (thread 0) issue the MMAs once
+//                the epilogue has released TMEM.  The packed samples arrive by cp.async one whole
+//                segment ahead, into a ring whose slots each thread fills and empties itself;
+//                segments alternate between two halves of TMEM, so the MMAs of the next one run
+//                while the epilogue still reads this one;
 //   warps 4-11 : epilogue; warp 4 + 4h + q reads TMEM lane quarter q of the tiles j = h (mod 2),
 //                adds the DC correction and stores each bin's 32 pixels as one coalesced row.
-// mbarriers `full` (MMAs of a segment complete: TMEM readable, A/B reusable) and `free` (the 8
-// epilogue warps finished reading TMEM), with bounded waits as in the fused pass.
+// mbarriers per half: `full` (MMAs of a segment complete: TMEM readable, A/B reusable) and `free` (the
+// 8 epilogue warps finished reading it), with bounded waits as in the fused pass.
+//
+// Bound: HBM, 4.0 GB for 4 windows of 128 x 1024 x 1536 at 56 bins (620 us at the copy rate).  With the
+// samples staged through registers, one round of 24 KB ahead, the loaders took 13 us per 512-pixel
+// segment and the epilogue, which could not start on the next one before they were done, 7: 1466 us in
+// all, 981 now (4.1 TB/s; 4 windows of 64 x 768^2 at 28 bins 266 -> 213).  The ring keeps 49 KB in
+// flight all the time and hides the loads completely; what is left is the epilogue's stores and the
+// hand-over of A between segments.
 //
 // One launch can serve several acquisitions of the same window length and sample format (the
 // batched uneven acquisitions): each is a job with its own ring, W, planes and geometry, and the
@@ -48,7 +58,18 @@ using tcb::wait_or_abort;
 constexpr int kSegLoaders  = 128; // warps 0-3
 constexpr int kSegEpilogue = 256; // warps 4-11
 constexpr int kSegThr      = kSegLoaders + kSegEpilogue;
-constexpr int kSegABytes   = 131072; // A operand: seg tiles x T frames x 128 pixels, f16 (seg T <= 512)
+constexpr int kSegCols     = 256; // TMEM columns of a segment: two segments in turn
+constexpr int kSegTF       = 256; // tiles x frames of a segment: A holds 256 bytes of f16 for each
+constexpr int kSegItems    = kSegTF * 4 / kSegLoaders; // a loader's items of 32 samples per segment
+// The loaders' ring: one slot more than a segment's items; a slot's pitch is an odd multiple of 16
+// bytes, so that neighbouring threads' 16-byte reads touch different banks.
+template <int FMT> struct SegRing {
+  static constexpr int kPitch = FMT == HF_MONO12P ? 48 : 80;
+  static constexpr int kSlots = kSegItems + 1;
+  static constexpr int kBytes = kSlots * kSegLoaders * kPitch;
+};
+constexpr int kSegABytes   = kSegTF * 256;
+constexpr int kUnitSlots   = 4; // unit indexes kept: one ahead of the loaders, one behind
 constexpr int kSegMaxN     = 128;    // MMA N (Nz <= 64)
 
 struct SegGeom {
@@ -98,18 +119,22 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
   // pointer
   uint8_t  *smem   = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t  *sA     = smem;                                        // g.seg tiles
-  uint8_t  *sB     = sA + kSegABytes;                             // hi [KA][N][128 B], then lo
-  float    *colsum = reinterpret_cast<float *>(sB + 2 * J.bpart_max); // [2][128], by window parity
-  int64_t  *foff   = reinterpret_cast<int64_t *>(colsum + 256);   // [T] frame offsets of the window
-  int64_t  *unitbuf = foff + 128;                                 // [2] unit of iteration k, by parity
-  uint64_t *mbar   = reinterpret_cast<uint64_t *>(unitbuf + 2);   // [0] full, [1] free
-  uint32_t *tslot  = reinterpret_cast<uint32_t *>(mbar + 2);
+  using RG         = SegRing<FMT>;
+  uint8_t  *sB     = sA + kSegABytes;                            // hi [KA][N][128 B], then lo
+  uint8_t  *ring   = sB + 2 * J.bpart_max;                        // [kSlots][kSegLoaders][kPitch] packed samples
+  float    *colsum = reinterpret_cast<float *>(ring + RG::kBytes); // [4][128], windows in turn
+  int64_t  *foff   = reinterpret_cast<int64_t *>(colsum + 512);   // [2][128] frame offsets, by window parity
+  int64_t  *unitbuf = foff + 256;                                 // [kUnitSlots] unit of iteration k
+  uint64_t *mbar   = reinterpret_cast<uint64_t *>(unitbuf + kUnitSlots); // full[2], free[2]
+  uint32_t *tslot  = reinterpret_cast<uint32_t *>(mbar + 4);
   int      *abort_flag = reinterpret_cast<int *>(tslot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    tc::mbar_init(&mbar[0], 2); // the MMA commit + the issuing thread's release arrive
-    tc::mbar_init(&mbar[1], kSegEpilogue / 32);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&mbar[i], 2); // the MMA commit + the issuing thread's release arrive
+      tc::mbar_init(&mbar[2 + i], kSegEpilogue / 32);
+    }
     *abort_flag = 0;
     tc::mbar_fence_init();
   }
@@ -121,43 +146,102 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
   const uint32_t tbase  = *tslot;
   volatile int  *abortv = abort_flag;
   const int64_t  nunits = J.nunits;
+  // segment k uses TMEM half k & 1 and the barriers of that half, in phase (k >> 1) & 1
+  uint64_t *const full = mbar, *const free_ = mbar + 2;
+  const auto      phase = [](int k) { return (uint32_t)((k >> 1) & 1); };
 
   if (tid < kSegLoaders) {
     // ------------------------------------------------------------------ loader / MMA warps
-    int k = 0, cur_ji = -1, cur_w = -1, wpar = 1;
-    for (;; ++k) {
-      if (k > 0) // MMAs of the previous segment done: A and B may be overwritten
-        wait_or_abort(&mbar[0], (uint32_t)((k - 1) & 1), abortv, J.status, 31);
-      if (tid == 0)
-        unitbuf[k & 1] = atomicAdd(J.counter, 1);
+    using GL         = GroupLoad<FMT>;
+    constexpr int IT = kSegItems;
+    int           k = 0, cur_ji = -1, cur_w = -1, wpar = 1; // window of B and its DC corrections
+    int           nxt_ji = -1, nxt_w = -1, npar = 1;        // window of the segment being fetched
+    int           fill = 0, drain = 0;                      // this thread's ring slots
+    uint8_t      *mine = ring + (size_t)tid * RG::kPitch;
+    // a segment of the work list: job, window, row, first tile, tiles
+    struct Seg {
+      int ji, w, r, j0, nt;
+    };
+    const auto decode = [&](int64_t u) {
+      Seg           q;
+      q.ji              = job_of(J, u);
+      const SegJob &a   = J.job[q.ji];
+      const int64_t uj  = u - a.unit0;
+      q.w               = (int)(uj / ((int64_t)a.H * a.g.spr));
+      const int64_t rem = uj - (int64_t)q.w * a.H * a.g.spr;
+      q.r               = (int)(rem / a.g.spr);
+      q.j0              = (int)(rem - (int64_t)q.r * a.g.spr) * a.g.seg;
+      q.nt              = min(a.g.seg, a.W / 128 - q.j0);
+      return q;
+    };
+    // work item `it` of a segment = (tile, frame t, 32-pixel group); consecutive threads take the four
+    // groups of one frame row, so each quad reads 128 contiguous pixels.  One commit group per call.
+    const auto fetch = [&](const Seg &q, const int64_t *fo, int it) {
+      if (it < q.nt * T * 4) {
+        const SegJob  &a = J.job[q.ji];
+        const int      j = it / (T * 4), t = (it >> 2) % T, grp = it & 3;
+        const uint8_t *src = a.ring.base + fo[t] + ((int64_t)q.r * a.W + 128 * (q.j0 + j) + 32 * grp) * GL::kBytes / 32;
+        const uint32_t dst = tc::smem_u32(mine + (size_t)fill * kSegLoaders * RG::kPitch);
+#pragma unroll
+        for (int i = 0; i < GL::kBytes / 16; ++i)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      fill = fill + 1 == RG::kSlots ? 0 : fill + 1;
+    };
+    const auto offsets = [&](const Seg &q, int64_t *fo) { // frame offsets of the segment's window
+      const SegJob &a = J.job[q.ji];
+      for (int t = tid; t < T; t += kSegLoaders)
+        fo[t] = a.ring.frame(q.w, t) - a.ring.base;
+    };
+    if (tid == 0)
+      unitbuf[0] = atomicAdd(J.counter, 1);
+    named_bar(1, kSegLoaders);
+    Seg nxt{};
+    if (unitbuf[0] < nunits) { // the first segment's samples
+      nxt    = decode(unitbuf[0]);
+      nxt_ji = nxt.ji, nxt_w = nxt.w, npar = 0;
+      offsets(nxt, foff);
       named_bar(1, kSegLoaders);
-      const int64_t u = unitbuf[k & 1];
+#pragma unroll
+      for (int i = 0; i < IT; ++i)
+        fetch(nxt, foff, i * kSegLoaders + tid);
+    }
+    for (;; ++k) {
+      const int64_t u = unitbuf[k % kUnitSlots];
+      if (tid == 0)
+        unitbuf[(k + 1) % kUnitSlots] = u < nunits ? (int64_t)atomicAdd(J.counter, 1) : nunits;
+      if (k > 0) // MMAs of the previous segment done: A and B may be overwritten
+        wait_or_abort(&full[(k - 1) & 1], phase(k - 1), abortv, J.status, 31);
+      named_bar(1, kSegLoaders);
       if (u >= nunits) { // no segments left: complete this phase empty so that the epilogue ends too
         if (tid == 0) {
-          // only after the epilogue has released the previous segment (see the fused pass)
-          if (k > 0)
-            wait_or_abort(&mbar[1], (uint32_t)((k - 1) & 1), abortv, J.status, 34);
-          mbar_arrive_cnt(&mbar[0], 2);
+          // only after the epilogue has released the half's last segment (see the fused pass)
+          if (k > 1)
+            wait_or_abort(&free_[k & 1], phase(k - 2), abortv, J.status, 34);
+          mbar_arrive_cnt(&full[k & 1], 2);
         }
         break;
       }
-      const int     ji  = job_of(J, u);
-      const SegJob &a   = J.job[ji];
+      const Seg     cur = nxt;
+      const SegJob &a   = J.job[cur.ji];
       const SegGeom g   = a.g;
-      const int     bpart = KA * g.N * 128;
-      const int64_t uj  = u - a.unit0;
-      const int     w   = (int)(uj / ((int64_t)a.H * g.spr));
-      const int64_t rem = uj % ((int64_t)a.H * g.spr);
-      const int     r = (int)(rem / g.spr), sg = (int)(rem % g.spr);
-      const int     j0 = sg * g.seg, nt = min(g.seg, a.W / 128 - j0);
-      const bool    new_w = w != cur_w || ji != cur_ji;
-      if (new_w) { // per window: frame offsets and B = (Wh, Wl) rows n = 2 bin + {re, im}
-        cur_ji = ji;
-        cur_w  = w;
-        wpar ^= 1;
-        for (int t = tid; t < T; t += kSegLoaders)
-          foff[t] = a.ring.frame(w, t) - a.ring.base;
-        const float2 *wm = a.wmat + (int64_t)w * a.wmat_stride;
+      const int     bpart = KA * g.N * 128, nt = cur.nt;
+      const bool    new_w = cur.w != cur_w || cur.ji != cur_ji;
+      const int64_t un    = unitbuf[(k + 1) % kUnitSlots];
+      const bool    more  = un < nunits;
+      if (more)
+        nxt = decode(un);
+      const bool nxt_new = more && (nxt.w != nxt_w || nxt.ji != nxt_ji);
+      if (nxt_new) {
+        nxt_ji = nxt.ji, nxt_w = nxt.w, npar ^= 1;
+        offsets(nxt, foff + npar * 128);
+      }
+      if (new_w) { // per window: B = (Wh, Wl) rows n = 2 bin + {re, im}
+        cur_ji = cur.ji;
+        cur_w  = cur.w;
+        wpar   = (wpar + 1) & 3;
+        const float2 *wm = a.wmat + (int64_t)cur.w * a.wmat_stride;
         for (int e = tid; e < g.N * (T / 8); e += kSegLoaders) {
           const int n = e / (T / 8), c8 = e % (T / 8); // one 16-byte chunk = 8 frames
           __half    hv[8], lv[8];
@@ -176,57 +260,46 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
           *reinterpret_cast<uint4 *>(sB + off)         = *reinterpret_cast<const uint4 *>(hv);
           *reinterpret_cast<uint4 *>(sB + bpart + off) = *reinterpret_cast<const uint4 *>(lv);
         }
-        named_bar(1, kSegLoaders); // frame offsets visible to every loader
       }
+      if (nxt_new)
+        named_bar(1, kSegLoaders); // its frame offsets are visible to every loader
       // A: tile j = pixels [128 (j0 + j), +128) of row r; element (m, t) at
       //    (m/64)*(128 T) + (t/8)*1024 + (t%8)*128 + ((m%64/8) ^ (t%8))*16 + (m%8)*2.
-      //    Work item `it` = (tile j, frame t, 32-pixel group grp); consecutive threads take the four
-      //    groups of one frame row, so each quad reads 128 contiguous pixels.  The packed words of
-      //    round rd + 1 are loaded before round rd is unpacked.
+      //    Item i of the next segment is fetched before item i of this one is unpacked.
       {
-        using GL          = GroupLoad<FMT>;
-        constexpr int U   = GL::kPerRound;
-        constexpr int NR  = (kSegABytes / 256 * 4 / kSegLoaders + U - 1) / U; // rounds at most
-        const int  nitems = nt * T * 4;
-        uint32_t   raw[2][U][GL::kWords];
         const float magic = 8388608.f + a.shift; // x - shift exactly: (2^23 + x) - (2^23 + shift)
-        auto load_round = [&](int rd, uint32_t (&dst)[U][GL::kWords]) {
+#pragma unroll 2
+        for (int i = 0; i < IT; ++i) {
+          const int it = i * kSegLoaders + tid;
+          if (more)
+            fetch(nxt, foff + npar * 128, it);
+          else
+            asm volatile("cp.async.commit_group;" ::: "memory");
+          asm volatile("cp.async.wait_group %0;" ::"n"(IT) : "memory"); // this thread's item i has landed
+          const uint4 *src = reinterpret_cast<const uint4 *>(mine + (size_t)drain * kSegLoaders * RG::kPitch);
+          drain            = drain + 1 == RG::kSlots ? 0 : drain + 1;
+          if (it >= nt * T * 4)
+            continue;
+          const int j = it / (T * 4), t = (it >> 2) % T, grp = it & 3;
+          uint32_t  raw[GL::kWords], v[32];
 #pragma unroll
-          for (int uu = 0; uu < U; ++uu) {
-            const int it = (rd * U + uu) * kSegLoaders + tid;
-            if (it < nitems) {
-              const int j = it / (T * 4), t = (it >> 2) % T, grp = it & 3;
-              GL::raw(a.ring.base + foff[t] + ((int64_t)r * a.W + 128 * (j0 + j) + 32 * grp) * GL::kBytes / 32,
-                      dst[uu]);
-            }
+          for (int q = 0; q < GL::kWords / 4; ++q) {
+            const uint4 x = src[q];
+            raw[4 * q] = x.x, raw[4 * q + 1] = x.y, raw[4 * q + 2] = x.z, raw[4 * q + 3] = x.w;
           }
-        };
-        load_round(0, raw[0]);
+          GL::unpack(raw, v);
+          uint8_t *tile = sA + j * TILE;
 #pragma unroll
-        for (int rd = 0; rd < NR; ++rd) {
-          if (rd + 1 < NR)
-            load_round(rd + 1, raw[(rd + 1) & 1]);
+          for (int q = 0; q < 4; ++q) {
+            const int m0 = 32 * grp + 8 * q;
+            __half2   h[4];
 #pragma unroll
-          for (int uu = 0; uu < U; ++uu) {
-            const int it = (rd * U + uu) * kSegLoaders + tid;
-            if (it >= nitems)
-              continue;
-            const int j = it / (T * 4), t = (it >> 2) % T, grp = it & 3;
-            uint32_t  v[32];
-            GL::unpack(raw[rd & 1][uu], v);
-            uint8_t *tile = sA + j * TILE;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int m0 = 32 * grp + 8 * q;
-              __half2   h[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                h[i] = __floats2half2_rn(__uint_as_float(0x4B000000u | v[8 * q + 2 * i]) - magic,
-                                         __uint_as_float(0x4B000000u | v[8 * q + 2 * i + 1]) - magic);
-              const int chunk = (m0 & 63) >> 3;
-              uint8_t  *dst   = tile + (m0 >> 6) * (T * 128) + (t >> 3) * 1024 + (t & 7) * 128 + ((chunk ^ (t & 7)) << 4);
-              *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(h);
-            }
+            for (int e = 0; e < 4; ++e)
+              h[e] = __floats2half2_rn(__uint_as_float(0x4B000000u | v[8 * q + 2 * e]) - magic,
+                                       __uint_as_float(0x4B000000u | v[8 * q + 2 * e + 1]) - magic);
+            const int chunk = (m0 & 63) >> 3;
+            uint8_t  *dst   = tile + (m0 >> 6) * (T * 128) + (t >> 3) * 1024 + (t & 7) * 128 + ((chunk ^ (t & 7)) << 4);
+            *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(h);
           }
         }
       }
@@ -244,8 +317,8 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
       tc::fence_proxy_async_smem();
       named_bar(1, kSegLoaders);
       if (tid == 0) {
-        if (k > 0) // the epilogue has read the previous segment out of TMEM
-          wait_or_abort(&mbar[1], (uint32_t)((k - 1) & 1), abortv, J.status, 32);
+        if (k > 1) // the epilogue has read segment k - 2 out of this half
+          wait_or_abort(&free_[k & 1], phase(k - 2), abortv, J.status, 32);
         tc::fence_after_sync();
         if (!*abortv) {
           const uint32_t idesc = tc::idesc_f16(128, g.N, true, false);
@@ -256,11 +329,11 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
               const uint64_t ad   = tc::sw128_desc(tc::smem_u32(sA + j * TILE + ks * 2048), T * 128, 1024);
               const uint64_t bd =
                   tc::sw128_desc(tc::smem_u32(sB + part * bpart + (ks >> 2) * g.N * 128 + (ks & 3) * 32), 16, 1024);
-              tc::mma_f16(tbase + (uint32_t)(j * g.ncol), ad, bd, idesc, s > 0 ? 1u : 0u);
+              tc::mma_f16(tbase + (uint32_t)((k & 1) * kSegCols + j * g.ncol), ad, bd, idesc, s > 0 ? 1u : 0u);
             }
         }
-        tc::mma_commit(&mbar[0]);
-        mbar_arrive(&mbar[0]); // release: the unit index, B and the DC correction are in place
+        tc::mma_commit(&full[k & 1]);
+        mbar_arrive(&full[k & 1]); // release: the unit index, B and the DC correction are in place
       }
     }
   } else {
@@ -268,9 +341,9 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
     const int e = warp - 4, q = warp & 3, half = e >> 2;
     int       k = 0, cur_ji = -1, cur_w = -1, wpar = 1;
     for (;; ++k) {
-      wait_or_abort(&mbar[0], (uint32_t)(k & 1), abortv, J.status, 33);
+      wait_or_abort(&full[k & 1], phase(k), abortv, J.status, 33);
       tc::fence_after_sync();
-      const int64_t u = unitbuf[k & 1];
+      const int64_t u = unitbuf[k % kUnitSlots];
       if (u >= nunits || *abortv)
         break;
       const int     ji   = job_of(J, u);
@@ -285,7 +358,7 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
       if (w != cur_w || ji != cur_ji) {
         cur_ji = ji;
         cur_w  = w;
-        wpar ^= 1;
+        wpar   = (wpar + 1) & 3;
       }
       const float *cs   = colsum + wpar * 128;
       float2      *orow = a.out + (int64_t)w * a.out_win + (int64_t)r * a.out_row + 32 * q + lane;
@@ -297,7 +370,7 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
 #pragma unroll
           for (int gi = 0; gi < 4; ++gi)
             if (gi < ng)
-              tc::tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(j * g.ncol + 8 * (g0 + gi)), v[gi]);
+              tc::tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)((k & 1) * kSegCols + j * g.ncol + 8 * (g0 + gi)), v[gi]);
           tc::tmem_wait_ld();
 #pragma unroll
           for (int gi = 0; gi < 4; ++gi)
@@ -314,9 +387,10 @@ __global__ void __launch_bounds__(kSegThr, 1) band_seg_tc_kernel(const __grid_co
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0)
-        mbar_arrive(&mbar[1]);
+        mbar_arrive(&free_[k & 1]);
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) {
@@ -331,7 +405,7 @@ SegGeom seg_geom(int T, int W, int nz, int seg_cap) {
   SegGeom g{};
   g.N    = 16 * ((2 * nz + 15) / 16);
   g.ncol = g.N <= 32 ? 32 : (g.N <= 64 ? 64 : 128);
-  g.seg  = std::min({512 / g.ncol, kSegABytes / (T * 256), W / 128});
+  g.seg  = std::min({kSegCols / g.ncol, kSegTF / T, W / 128});
   if (seg_cap > 0)
     g.seg = std::min(g.seg, seg_cap);
   g.spr  = (W / 128 + g.seg - 1) / g.seg;
@@ -339,7 +413,8 @@ SegGeom seg_geom(int T, int W, int nz, int seg_cap) {
 }
 
 template <int FMT, int T> int launch_t(SegJobs &J, int max_ctas, cudaStream_t s) {
-  const size_t smem = 1024 + (size_t)kSegABytes + 2 * (size_t)J.bpart_max + 256 * 4 + 128 * 8 + 2 * 8 + 2 * 8 + 16;
+  const size_t smem = 1024 + (size_t)kSegABytes + 2 * (size_t)J.bpart_max + SegRing<FMT>::kBytes + 512 * 4 +
+                      256 * 8 + kUnitSlots * 8 + 4 * 8 + 16;
   HF_CUDA(cudaFuncSetAttribute(band_seg_tc_kernel<FMT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int cap  = max_ctas > 0 ? std::min(max_ctas, sm_count()) : sm_count();
   const int grid = (int)std::min<int64_t>(J.nunits, cap);
