@@ -20,7 +20,7 @@
 //    strips per transform, the next group's strips arriving by cp.async into a third buffer while
 //    the current group is transformed, and the per-sub-aperture fftshift fused into the store.
 //  - shk_roi_mean_kernel, shk_peak_kernel (first maximum + parabolic refinement, one CTA per map),
-//    shk_slopes_kernel and shk_zfit_kernel (one thread each: the reference's float32 sequences),
+//    shk_slopes_kernel (one thread) and shk_zfit_kernel (one warp): the reference's float32 sequences,
 //    shk_zernike_phase_kernel, shk_correct_phase_kernel, shk_wrap2pi_kernel.
 #include <algorithm>
 #include <cfloat>
@@ -644,75 +644,108 @@ struct ZFit {
 };
 
 // The data-dependent half of ZernikeFromSlopes::execute (zernike_from_slopes.cc:246-277) in one
-// thread, with the host's float32 operations made explicit (no contraction) so that the result is
+// warp, with the host's float32 operations made explicit (no contraction) so that the result is
 // the reference's bit for bit: gts[i] += gx_i sx + gy_i sy over the active samples in row-major
 // order, then Gaussian elimination with partial pivoting and back substitution.
-__device__ void zfit_solve(const ZFit &z, const float *g, const float *slopes, float *coeffs) {
-  float m[kShkMaxModes][kShkMaxModes], rhs[kShkMaxModes], sol[kShkMaxModes];
-  const int n = z.nobs;
-  for (int i = 0; i < n; ++i) {
-    rhs[i] = 0.f, sol[i] = 0.f;
-    for (int j = 0; j < n; ++j)
-      m[i][j] = z.gtg[i][j];
-  }
-  for (int s = 0; s < z.count; ++s) {
-    const float *gs = g + (size_t)s * 2 * kShkMaxModes; // [gx[0..8], gy[0..8]] (mean removed); NaN marks inactive
-    if (isnan(gs[0]) && n > 0)
-      continue;
-    const float sx = slopes[2 * s], sy = slopes[2 * s + 1];
-    for (int i = 0; i < n; ++i)
-      rhs[i] = __fadd_rn(rhs[i], __fadd_rn(__fmul_rn(gs[i], sx), __fmul_rn(gs[kShkMaxModes + i], sy)));
+// One warp: lane i sums the right-hand side of mode i and owns row i of the system, so every element
+// takes the host's operations in the host's order (a single thread with the system in local memory
+// took 23 us for 25 samples and 3 modes).
+constexpr int kZfitChunk = 64; // samples staged at a time
+__global__ void __launch_bounds__(32) shk_zfit_kernel(ZFit z, const float *g, const float *slopes, float *coeffs,
+                                                      float *cumulative) {
+  __shared__ float sg[kZfitChunk * 2 * kShkMaxModes], ss[kZfitChunk * 2];
+  constexpr int    N    = kShkMaxModes;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x, n = z.nobs;
+  float     row[N], rhs = 0.f;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    row[j] = lane < n && j < n ? z.gtg[lane < N ? lane : 0][j] : 0.f;
+  for (int s0 = 0; s0 < z.count; s0 += kZfitChunk) {
+    const int ns = min(kZfitChunk, z.count - s0);
+    for (int e = lane; e < ns * 2 * N; e += 32)
+      sg[e] = g[(size_t)s0 * 2 * N + e];
+    for (int e = lane; e < ns * 2; e += 32)
+      ss[e] = slopes[2 * s0 + e];
+    __syncwarp();
+    if (lane < n)
+      for (int s = 0; s < ns; ++s) {
+        const float *gs = sg + s * 2 * N; // [gx[0..8], gy[0..8]] (mean removed); NaN marks inactive
+        if (!isnan(gs[0]))
+          rhs = __fadd_rn(rhs, __fadd_rn(__fmul_rn(gs[lane], ss[2 * s]), __fmul_rn(gs[N + lane], ss[2 * s + 1])));
+      }
+    __syncwarp();
   }
   bool singular = false;
-  for (int c = 0; c < n && !singular; ++c) {
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    if (c >= n || singular)
+      continue;
     int   piv = c;
-    float bv  = fabsf(m[c][c]);
-    for (int r = c + 1; r < n; ++r)
-      if (fabsf(m[r][c]) > bv)
-        bv = fabsf(m[r][c]), piv = r;
+    float bv  = fabsf(__shfl_sync(kAll, row[c], c));
+#pragma unroll
+    for (int r = c + 1; r < N; ++r) {
+      const float v = fabsf(__shfl_sync(kAll, row[c], r));
+      if (r < n && v > bv)
+        bv = v, piv = r;
+    }
     if (bv < 1e-12f) {
       singular = true;
-      break;
+      continue;
     }
-    if (piv != c) {
-      for (int j = 0; j < n; ++j) {
-        const float t = m[piv][j];
-        m[piv][j] = m[c][j], m[c][j] = t;
+    const int from = lane == c ? piv : (lane == piv ? c : lane); // rows c and piv exchanged
+    rhs = __shfl_sync(kAll, rhs, from);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      row[j] = __shfl_sync(kAll, row[j], from);
+    const float pv = __shfl_sync(kAll, row[c], c), f = row[c];
+    const float pr = __fdiv_rn(__shfl_sync(kAll, rhs, c), pv);
+    if (lane == c)
+      rhs = pr;
+    else if (lane > c)
+      rhs = __fsub_rn(rhs, __fmul_rn(f, pr));
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const float pj = __fdiv_rn(__shfl_sync(kAll, row[j], c), pv);
+      if (j >= c && j < n) {
+        if (lane == c)
+          row[j] = pj;
+        else if (lane > c)
+          row[j] = __fsub_rn(row[j], __fmul_rn(f, pj));
       }
-      const float t = rhs[piv];
-      rhs[piv] = rhs[c], rhs[c] = t;
-    }
-    const float pv = m[c][c];
-    for (int j = c; j < n; ++j)
-      m[c][j] = __fdiv_rn(m[c][j], pv);
-    rhs[c] = __fdiv_rn(rhs[c], pv);
-    for (int r = c + 1; r < n; ++r) {
-      const float f = m[r][c];
-      for (int j = c; j < n; ++j)
-        m[r][j] = __fsub_rn(m[r][j], __fmul_rn(f, m[c][j]));
-      rhs[r] = __fsub_rn(rhs[r], __fmul_rn(f, rhs[c]));
     }
   }
-  if (!singular)
-    for (int r = n - 1; r >= 0; --r) {
-      float v = rhs[r];
-      for (int c = r + 1; c < n; ++c)
-        v = __fsub_rn(v, __fmul_rn(m[r][c], sol[c]));
-      sol[r] = v;
-    }
-  for (int i = 0; i < z.nidx; ++i)
-    coeffs[i] = 0.f;
-  for (int i = 0; i < n; ++i)
-    coeffs[z.pos[i]] = singular ? 0.f : __fmul_rn(sol[i], z.rad_per_m);
-}
-
-__global__ void shk_zfit_kernel(ZFit z, const float *g, const float *slopes, float *coeffs, float *cumulative) {
-  if (blockIdx.x != 0 || threadIdx.x != 0)
+  float sol[N];
+#pragma unroll
+  for (int r = N - 1; r >= 0; --r) {
+    float v = rhs;
+#pragma unroll
+    for (int c = r + 1; c < N; ++c)
+      if (c < n)
+        v = __fsub_rn(v, __fmul_rn(row[c], sol[c]));
+    sol[r] = __shfl_sync(kAll, v, r);
+  }
+  if (lane != 0)
     return;
-  zfit_solve(z, g, slopes, coeffs);
-  if (cumulative)
-    for (int i = 0; i < z.nidx; ++i)
-      cumulative[i] += coeffs[i];
+  float out[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    out[i] = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < n && !singular) {
+#pragma unroll
+      for (int q = 0; q < N; ++q)
+        if (q == z.pos[i])
+          out[q] = __fmul_rn(sol[i], z.rad_per_m);
+    }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < z.nidx) {
+      coeffs[i] = out[i];
+      if (cumulative)
+        cumulative[i] += out[i];
+    }
 }
 
 struct ZModes {
@@ -741,7 +774,10 @@ __device__ __forceinline__ float zernike_value(int noll, float x, float y) {
 // centred on the grid.  `accumulate` adds the phase to `phase` (the cumulative map of repeated
 // passes) instead of overwriting it.
 // Rows over blockIdx.y, columns over the threads: no index division per pixel.
-__global__ void shk_zernike_phase_kernel(const float *coeffs, ZModes zm, int ny, int nx, float *phase, float *cumulative) {
+// `lens`: instead of the map, lens exp(-i phase) goes to `folded` (the correction in the Fresnel lens
+// that the row pass multiplies by).
+__global__ void shk_zernike_phase_kernel(const float *coeffs, ZModes zm, int ny, int nx, float *phase, float *cumulative,
+                                         const float2 *lens, float2 *folded) {
   const float cy = ((float)ny - 1.0f) * 0.5f, cx = ((float)nx - 1.0f) * 0.5f;
   const float r  = 0.5f * (float)(ny < nx ? ny : nx);
   float       c[kShkMaxModes];
@@ -756,11 +792,30 @@ __global__ void shk_zernike_phase_kernel(const float *coeffs, ZModes zm, int ny,
       for (int m = 0; m < zm.n; ++m)
         ph += c[m] * zernike_value(zm.idx[m], x, y);
       const int64_t i = (int64_t)yi * nx + xi;
-      phase[i]        = ph;
+      if (lens != nullptr) {
+        float sv, cv;
+        sincosf(ph, &sv, &cv);
+        const float2 l = lens[i];
+        folded[i]      = make_float2(l.x * cv + l.y * sv, l.y * cv - l.x * sv);
+        continue;
+      }
+      phase[i] = ph;
       if (cumulative)
         cumulative[i] += ph;
     }
   }
+}
+
+int launch_zernike_phase(const float *coeffs, const int *indexes, int n_indexes, int ny, int nx, float *phase,
+                         float *cumulative, const float2 *lens, float2 *folded, cudaStream_t s) {
+  ZModes zm{};
+  zm.n = n_indexes;
+  for (int i = 0; i < n_indexes; ++i)
+    zm.idx[i] = indexes[i];
+  const dim3 zg((unsigned)std::min(4, (nx + 255) / 256), (unsigned)std::min(ny, 65535));
+  shk_zernike_phase_kernel<<<zg, 256, 0, s>>>(coeffs, zm, ny, nx, phase, cumulative, lens, folded);
+  note_launch();
+  return launch_status("shk_zernike_phase_kernel");
 }
 
 // correct_phase_cf32_kernel / correct_phase_f32_to_cf32_kernel (correct_phase.cu:76-106):
@@ -1289,7 +1344,7 @@ void release(hf_zernike_fit *f) {
   delete f;
 }
 
-// Host copy of the fit (the reference runs it on the host): same sequence as zfit_solve.
+// Host copy of the fit (the reference runs it on the host): same sequence as shk_zfit_kernel.
 void zfit_host(const hf_zernike_fit *f, const float *slopes, float *coeffs) {
   const ZFit &z = f->z;
   const int   n = z.nobs;
@@ -1470,14 +1525,7 @@ int hf_zernike_phase(const float *coeffs, const int *indexes, int n_indexes, int
   HF_TRY(check_indexes(indexes, n_indexes, "ZernikePhaseFactory inference error"));
   HF_CHECK_ARG(ny > 0 && nx > 0, "ZernikePhaseFactory inference error: Resolution ny and nx must be greater than 0");
   HF_CHECK_ARG(coeffs != nullptr && phase != nullptr, "ZernikePhase: null argument");
-  ZModes zm{};
-  zm.n = n_indexes;
-  for (int i = 0; i < n_indexes; ++i)
-    zm.idx[i] = indexes[i];
-  const dim3 zg((unsigned)std::min(4, (nx + 255) / 256), (unsigned)std::min(ny, 65535));
-  shk_zernike_phase_kernel<<<zg, 256, 0, s>>>(coeffs, zm, ny, nx, phase, cumulative);
-  note_launch();
-  return launch_status("shk_zernike_phase_kernel");
+  return launch_zernike_phase(coeffs, indexes, n_indexes, ny, nx, phase, cumulative, nullptr, nullptr, s);
 }
 
 int hf_correct_phase(const void *in, int complex_input, const float *phase, int64_t planes, int height, int width,
@@ -1671,13 +1719,14 @@ int hf_autofocus_exec(hf_autofocus *a, const void *planes, const void *delayed, 
   clear_error();
   HF_CHECK_ARG(a != nullptr && planes != nullptr && corrected != nullptr, "Autofocus: null argument");
   const int64_t total = (int64_t)a->nz * a->H * a->W;
-  HF_TRY(hf::autofocus_begin(a, s));
+  HF_TRY(hf::autofocus_begin(a, true, s));
   for (int pass = 0; pass < a->n_iter; ++pass) {
     // pass 0 measures the current spectrum and corrects the delayed one; later passes measure and
     // correct their predecessor's output (graph_builder.cc:149-153)
     const void *cur = pass == 0 ? planes : corrected;
     const void *del = pass == 0 ? (delayed ? delayed : planes) : corrected;
     HF_TRY(hf::autofocus_measure(a, cur, s));
+    HF_TRY(hf::autofocus_phase(a, true, s));
     if (a->nidx > 0)
       HF_TRY(hf_correct_phase(del, 1, a->phase, a->nz, a->H, a->W, corrected, s));
     else if (del != corrected) // no Zernike orders: a zero phase map, E exp(-i 0) = E
@@ -1729,21 +1778,13 @@ __global__ void shk_causal_avg_kernel(float *x, float *hist, float *sum, int64_t
   }
 }
 
-// lens exp(-i phase): the correction folded into the Fresnel lens that the row pass multiplies by
-__global__ void shk_fold_lens_kernel(const float2 *lens, const float *phase, float2 *out, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    float sv, cv;
-    sincosf(phase[i], &sv, &cv);
-    const float2 l = lens[i];
-    out[i]         = make_float2(l.x * cv + l.y * sv, l.y * cv - l.x * sv);
-  }
-}
 } // namespace
 
-int autofocus_begin(hf_autofocus *a, cudaStream_t s) {
+int autofocus_begin(hf_autofocus *a, bool phase_sum, cudaStream_t s) {
   a->pass = 0;
   HF_CUDA(cudaMemsetAsync(a->cum_coeffs, 0, kShkMaxModes * sizeof(float), s));
-  HF_CUDA(cudaMemsetAsync(a->cum_phase, 0, (size_t)a->H * a->W * sizeof(float), s));
+  if (phase_sum)
+    HF_CUDA(cudaMemsetAsync(a->cum_phase, 0, (size_t)a->H * a->W * sizeof(float), s));
   return HF_OK;
 }
 
@@ -1762,22 +1803,22 @@ int autofocus_measure(hf_autofocus *a, const void *planes, cudaStream_t s) {
   if (a->ff) // in place: each pass reads its input only where it writes, or before it writes
     HF_TRY(hf_flatfield_exec(a->ff, a->m0, a->m0, s));
   HF_TRY(hf_shslopes_exec(a->sl, a->m0, a->slopes, nullptr, s));
-  if (a->nidx > 0) {
-    HF_TRY(hf_zernike_fit_exec(a->fit, a->slopes, a->coeffs, a->cum_coeffs, s));
-    HF_TRY(hf_zernike_phase(a->coeffs, a->idx, a->nidx, a->H, a->W, a->phase, a->cum_phase, s));
-  }
-  return HF_OK;
+  return a->nidx > 0 ? hf_zernike_fit_exec(a->fit, a->slopes, a->coeffs, a->cum_coeffs, s) : HF_OK;
+}
+
+int autofocus_phase(hf_autofocus *a, bool phase_sum, cudaStream_t s) {
+  return a->nidx > 0 ? launch_zernike_phase(a->coeffs, a->idx, a->nidx, a->H, a->W, a->phase,
+                                            phase_sum ? a->cum_phase : nullptr, nullptr, nullptr, s)
+                     : HF_OK;
 }
 
 int autofocus_correct(hf_autofocus *a, const void *planes, void *out, cudaStream_t s) {
   return hf_correct_phase(planes, 1, a->phase, a->nz, a->H, a->W, out, s);
 }
 
+// The map of the last measurement goes straight into the lens (needs at least one order).
 int autofocus_fold_lens(hf_autofocus *a, const float2 *lens, float2 *out, cudaStream_t s) {
-  const int64_t n = (int64_t)a->H * a->W;
-  shk_fold_lens_kernel<<<grid_1d(n), 256, 0, s>>>(lens, a->phase, out, n);
-  note_launch();
-  return launch_status("shk_fold_lens_kernel");
+  return launch_zernike_phase(a->coeffs, a->idx, a->nidx, a->H, a->W, nullptr, nullptr, lens, out, s);
 }
 
 int autofocus_set_z(hf_autofocus *a, float z, cudaStream_t s) { return hf_stfd_set_z(a->stfd, z, s); }

@@ -7,14 +7,15 @@
 
 namespace hf {
 
-// Zeroes the coefficients and phase accumulated over the passes of one spectrum.
-int autofocus_begin(hf_autofocus *a, cudaStream_t s);
-// One measurement: sub-aperture M0, slopes, Zernike fit and phase map (kept as the pass's phase
-// and added to the accumulated ones); `planes` is [nz][H][W] complex64.
+// Zeroes the coefficients (and with `phase_sum` the phase) accumulated over the passes of one spectrum.
+int autofocus_begin(hf_autofocus *a, bool phase_sum, cudaStream_t s);
+// One measurement: sub-aperture M0, slopes and Zernike fit; `planes` is [nz][H][W] complex64.
 int autofocus_measure(hf_autofocus *a, const void *planes, cudaStream_t s);
-// out = planes exp(-i phase) with the last measured phase (in place allowed).
+// The phase map of the last measurement (with `phase_sum` also added to the accumulated one).
+int autofocus_phase(hf_autofocus *a, bool phase_sum, cudaStream_t s);
+// out = planes exp(-i phase) with the last phase map (in place allowed).
 int autofocus_correct(hf_autofocus *a, const void *planes, void *out, cudaStream_t s);
-// out = lens exp(-i phase): the last measured correction folded into a [H][W] lens.
+// out = lens exp(-i phase): the last measurement folded into a [H][W] lens, without a phase map.
 int autofocus_fold_lens(hf_autofocus *a, const float2 *lens, float2 *out, cudaStream_t s);
 // A new propagation distance: rebuilds the short-time Fresnel input lens.
 int autofocus_set_z(hf_autofocus *a, float z, cudaStream_t s);

@@ -341,11 +341,13 @@ static int phase_after_band(hf_plan *p, int nwin, float *out, cudaStream_t s, bo
         float2            *planes = p->band + w * win_px;
         hf_autofocus      *a      = two && (w & 1) ? p->af2 : p->af;
         const cudaStream_t q      = two && (w & 1) ? p->af_side : s;
-        HF_TRY(autofocus_begin(a, q));
+        HF_TRY(autofocus_begin(a, false, q));
         for (int pass = 0; pass < autofocus_passes(a); ++pass) {
           HF_TRY(autofocus_measure(a, planes, q));
-          if (pass + 1 < autofocus_passes(a))
+          if (pass + 1 < autofocus_passes(a)) {
+            HF_TRY(autofocus_phase(a, false, q));
             HF_TRY(autofocus_correct(a, planes, planes, q));
+          }
         }
         HF_TRY(autofocus_fold_lens(a, p->lens, p->lens_af + (int64_t)w * p->P, q));
         HF_CUDA(cudaMemcpyAsync(p->af_coeff + 9 * w, autofocus_cumulative_coeffs(a), 9 * sizeof(float),
