@@ -3,7 +3,7 @@
 //
 // G' = (X - 2048)^T (X - 2048) with X = [T][P] 12-bit samples: (x - 2048) is exact in f16, the
 // products are exact in the f32 accumulator, and the shift is undone in float64 by the shared
-// finalize kernel (k_pca.cu) from exact integer frame sums.  Per CTA: a ring of 4 shared-memory
+// finalize kernel (k_cov_fp32.cu) from exact integer frame sums.  Per CTA: a ring of 4 shared-memory
 // stages of 128 pixels x T frames in the canonical K-major 128-byte-swizzled layout (rows = frames,
 // K = pixels).  All threads unpack the next stage while the tensor core consumes the previous ones;
 // one thread issues M = N = T, K = 16 MMAs (A and B are the same tile) into a TMEM accumulator and
@@ -166,11 +166,12 @@ __global__ void __launch_bounds__(128) cov_tc_kernel(CovArgs a, int *status) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// Exact integer variant for samples of at most 12 bits: x - shift = 64 h + l with h in [-32, 31],
-// l in [0, 63] (both int8).  The stage of a 128-pixel tile holds 2 rows (h, l) per frame, K-major;
-// kind::i8 MMAs accumulate D = Z Z^T of a window's 2T rows Z in int32 TMEM columns, and
-// G' = 4096 HH + 64 (HL + LH) + LL is folded into a per-window int64 accumulator with integer
-// atomics (exact, so the result does not depend on their order).
+// Exact integer variant for samples of at most 12 bits: x = 16 h + l with h in [0, 255], l in [0, 15]
+// (both unsigned bytes).  The stage of a 128-pixel tile holds 2 rows (h, l) per frame, K-major; kind::i8
+// MMAs accumulate D = Z Z^T of a window's 2T rows Z in 32-bit TMEM columns, and
+// G = 256 HH + 16 (HL + LH) + LL is folded into a per-window int64 accumulator with integer atomics
+// (exact, so the result does not depend on their order).  An entry of D grows by at most 255^2 per pixel
+// and the accumulators wrap, so a CTA of up to 65536 pixels leaves each one exact as an unsigned number.
 //  - A CTA owns a group of up to G consecutive windows, i.e. the frames w0*hop + [0, F) with
 //    F = T + (G - 1) hop, and stages every frame of the group once per tile.  G = 4 for T = 64
 //    windows that overlap on an 8-frame grid (hop 8..32); G = 1 otherwise (T = 32, 64, 128).
@@ -179,15 +180,17 @@ __global__ void __launch_bounds__(128) cov_tc_kernel(CovArgs a, int *status) {
 //    descriptor offset selects them.  T = 32 is one M = N = 64 MMA per K-step and T = 64 one
 //    M = N = 128; T = 128 takes M = 128 twice, N = 256 for the first 64 frames' rows and N = 128
 //    (the last 64 frames' columns) for the rest, since D is symmetric.
-//  - Packed samples travel global -> shared through a ring of per-thread cp.async copies, D tiles
-//    deep; each thread unpacks exactly the bytes it copied, so no barrier guards the raw ring.
-//    Before, single windows loaded through registers, one tile ahead, between two block barriers
-//    per tile: 97 us for one 64 x 1024^2 window (15 us of bytes) and 718 us for four 128 x 1536 x
-//    1024 ones.
-//  - The split needs no pixel value: for x in [0, 4096), x - 2048 = 64 ((x >> 6) - 32) + (x & 63),
-//    so the 6-bit fields of the packed stream are masked out in 16-bit lanes, packed to bytes with
-//    byte permutes and re-centred with one byte-wise subtraction; frame sums are 64 S(x >> 6) +
-//    S(x & 63) from byte dot products.  8-bit samples use x - 128 = 64 ((x >> 6) - 2) + (x & 63).
+//  - Packed samples travel global -> shared through a ring of per-warp cp.async copies, D tiles deep;
+//    each warp unpacks exactly the bytes it copied, so no block barrier guards the raw ring.  The lanes
+//    copy the warp's 8 frame runs in order: lanes that copied their own 32 pixels, 48 bytes apart,
+//    asked for every sector twice (3 % slower).
+//  - The split is byte selects and masks on the packed stream (two pixels are b0 | (b1 & 15) << 8 and
+//    b1 >> 4 | b2 << 4, so l and h are the halves of b0, b1 and b2 as it is): 12 instructions per 8
+//    pixels.  The order of the pixels along K is free as long as every frame has the same.  Splitting at
+//    6 bits around 2048, with the frame sums that undoing the shift needs, took 50 and bound the kernel.
+// Measured, loads through registers between block barriers -> copy ring -> byte split: one 64 x 1024^2
+// window 97 -> 48 -> 41 us (15 us of bytes), eight at hop 16 152 -> 149 -> 123, four of 128 x 1024 x 1536
+// 718 -> 400 -> 274 (82 us of bytes read once; their products alone take 137 at the nominal int8 rate).
 // Operand row r of a window holds frame 8 (r / 16) + r % 8, kind h when (r / 8) is even; the h-row
 // and l-row of a frame sit 8 lanes apart in one warp and are folded with a shuffle before the
 // integer atomics, which cover the upper triangle.
@@ -201,12 +204,6 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// 24 packed bits (two 12-bit pixels p0 | p1 << 12) -> 16-bit lanes of their low and high 6 bits
-__device__ __forceinline__ void split_pair12(uint32_t t, uint32_t &lo, uint32_t &hi) {
-  lo = (t & 0x3Fu) | ((t << 4) & 0x003F0000u);
-  hi = ((t >> 6) & 0x3Fu) | ((t >> 2) & 0x003F0000u);
 }
 
 template <int FMT, int T, int G, int HOP8> struct GroupCov {
@@ -243,13 +240,11 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *mbar, uint32_t parity, v
 
 template <int FMT, int T, int NG, int HOP8>
 __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT, T, NG, HOP8>::PER_SM)
-    cov_tc_group_kernel(FrameRing ring, int64_t P, int nwin, uint32_t ncols, unsigned long long *acc,
-                        unsigned long long *sums, int *status) {
+    cov_tc_group_kernel(FrameRing ring, int64_t P, int nwin, uint32_t ncols, unsigned long long *acc, int *status) {
   using G                = GroupCov<FMT, T, NG, HOP8>;
   constexpr int HOP      = 8 * HOP8;
   constexpr int M        = T == 32 ? 64 : 128; // MMA rows
   constexpr int NMB      = 2 * T / M;          // M-blocks
-  constexpr uint32_t kHS = FMT == HF_MONO12P ? 0x20202020u : 0x02020202u; // shift / 64 per byte
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t  *smem  = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u); // stays a shared-space pointer
   uint8_t  *raw   = smem + G::S * G::STG;
@@ -280,24 +275,30 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
 
   const int      f      = tid >> 2, grp = tid & 3;
   const bool     active = f < Fg;
-  const uint8_t *fbase  = active ? ring.frame(w0, f) : nullptr;
   uint8_t       *myraw  = raw + (size_t)tid * G::RB;
   // this thread's rows in the stage: frame f -> pair f / 8, row f % 8 of the pair's h and l atoms
   const int rr = f & 7, pr = f >> 3;
 
   const int64_t ntiles = (P + kTcPX - 1) / kTcPX;
-  auto issue = [&](int64_t tile, int slot) {
-    const int64_t p = tile * kTcPX + grp * 32;
-    if (active && tile < ntiles && p < P) {
-      const uint8_t *src = fbase + p * TcBpp<FMT>::num / TcBpp<FMT>::den;
-      uint8_t       *dst = myraw + (size_t)slot * G::NT * G::RB;
+  // A warp's 32 runs are 8 frames x 128 pixels; its lanes copy them in order, 16 bytes each
+  constexpr int  CI = G::RB / 16;
+  const uint8_t *csrc[CI];
 #pragma unroll
-      for (int i = 0; i < G::RB / 16; ++i)
-        cp_async16(dst + 16 * i, src + 16 * i);
-    }
+  for (int i = 0; i < CI; ++i) {
+    const int c = 32 * i + lane;
+    csrc[i]     = active ? ring.frame(w0, 8 * warp + c / (4 * CI)) + 16 * (c % (4 * CI)) : nullptr;
+  }
+  auto issue = [&](int64_t tile, int slot) {
+    uint8_t *dst = raw + (size_t)slot * G::NT * G::RB + (size_t)warp * 32 * G::RB + 16 * lane;
+    if (active && tile < ntiles)
+#pragma unroll
+      for (int i = 0; i < CI; ++i) {
+        const int run = (32 * i + lane) % (4 * CI) / CI; // of this frame, 32 pixels each
+        if (tile * kTcPX + 32 * run < P)
+          cp_async16(dst + 512 * i, csrc[i] + tile * (kTcPX * TcBpp<FMT>::num / TcBpp<FMT>::den));
+      }
     cp_async_commit();
   };
-  uint32_t sx = 0u, sl = 0u; // sums of the high and low 6-bit fields
   int      nj = 0;
   bool     ok = true;
   if (producer) {
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
     if (nj >= G::S) // the MMAs that read this stage S tiles ago are done
       w_ok = wait_or_abort(&mbar[s], (uint32_t)((nj / G::S) - 1) & 1u, abortv, status, 5);
     cp_async_wait<G::D - 1>();
+    __syncwarp(); // the warp's copies of this tile have landed
     const bool valid = active && tile * kTcPX + grp * 32 < P;
     if (w_ok && active) {
       uint32_t hw[8], lw[8];
@@ -324,30 +326,22 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
         }
         if constexpr (FMT == HF_MONO12P) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) { // 8 pixels from 3 words
+          for (int q = 0; q < 4; ++q) { // 8 pixels from 3 words: every third byte of the 12
             const uint32_t a0 = wv[3 * q], a1 = wv[3 * q + 1], a2 = wv[3 * q + 2];
-            uint32_t       l0, h0, l1, h1, l2, h2, l3, h3;
-            split_pair12(a0, l0, h0);
-            split_pair12(__funnelshift_r(a0, a1, 24), l1, h1);
-            split_pair12(__funnelshift_r(a1, a2, 16), l2, h2);
-            split_pair12(a2 >> 8, l3, h3);
-            lw[2 * q]     = __byte_perm(l0, l1, 0x6420);
-            lw[2 * q + 1] = __byte_perm(l2, l3, 0x6420);
-            hw[2 * q]     = __byte_perm(h0, h1, 0x6420);
-            hw[2 * q + 1] = __byte_perm(h2, h3, 0x6420);
+            const uint32_t b0 = __byte_perm(__byte_perm(a0, a1, 0x0630), a2, 0x5210);
+            const uint32_t b1 = __byte_perm(__byte_perm(a0, a1, 0x0741), a2, 0x6210);
+            const uint32_t b2 = __byte_perm(__byte_perm(a0, a1, 0x0052), a2, 0x7410);
+            lw[2 * q]     = b0 & 0x0F0F0F0Fu; // the four even pixels, then the four odd ones
+            hw[2 * q]     = ((b0 >> 4) & 0x0F0F0F0Fu) | ((b1 << 4) & 0xF0F0F0F0u);
+            lw[2 * q + 1] = (b1 >> 4) & 0x0F0F0F0Fu;
+            hw[2 * q + 1] = b2;
           }
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            lw[i] = wv[i] & 0x3F3F3F3Fu;
-            hw[i] = (wv[i] >> 6) & 0x03030303u;
+            lw[i] = wv[i] & 0x0F0F0F0Fu;
+            hw[i] = (wv[i] >> 4) & 0x0F0F0F0Fu;
           }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          sx    = __dp4a(hw[i], 0x01010101u, sx);
-          sl    = __dp4a(lw[i], 0x01010101u, sl);
-          hw[i] = __vsub4(hw[i], kHS);
         }
       } else {
 #pragma unroll
@@ -368,7 +362,7 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
     __syncwarp();
     if (lane == 0)
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(&fullb[s])) : "memory");
-    if (!w_ok || *abortv) {
+    if (__any_sync(0xFFFFFFFFu, !w_ok || *abortv)) {
       ok = false;
       break;
     }
@@ -392,7 +386,7 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
 #pragma unroll
             for (int mb = 0; mb < NMB; ++mb) { // block mb against the columns from its own first row on
               const uint64_t d = tc::sw128_desc(z + mb * M * 128 + ks * 32, 16, 1024);
-              tc::mma_i8(tbase + G::WCOL * wl + mb * 2 * T, d, d, tc::idesc_i8(M, 2 * T - mb * M, false, false),
+              tc::mma_i8(tbase + G::WCOL * wl + mb * 2 * T, d, d, tc::idesc_u8(M, 2 * T - mb * M, false, false),
                          (nj > 0 || ks > 0) ? 1u : 0u);
             }
         }
@@ -408,24 +402,13 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
   ok = __syncthreads_and(ok && !*abortv) != 0;
   tc::fence_after_sync();
 
-  // frame sums: the four runs of a frame are adjacent lanes; each window holding frame f gets it
-  unsigned long long fs = 64ull * sx + sl;
-  fs += __shfl_xor_sync(0xFFFFFFFFu, fs, 1);
-  fs += __shfl_xor_sync(0xFFFFFFFFu, fs, 2);
-  if (producer && active && grp == 0)
-    for (int wl = 0; wl < g; ++wl) {
-      const int t = f - wl * HOP;
-      if (t >= 0 && t < T)
-        atomicAdd(&sums[(int64_t)(w0 + wl) * T + t], fs);
-    }
-
   constexpr int NQ = G::NT / 128; // complete warp quads: each reads all 128 TMEM lanes
   if (nj > 0 && ok && warp < 4 * NQ) {
     const int q  = warp & 3;
     // operand row of this lane within its M-block; M = 64 keeps row m in TMEM lane 32 (m / 16) + m % 16
     const int       r    = M == 64 ? 16 * q + (lane & 15) : 32 * q + lane;
     const bool      is_h = ((r >> 3) & 1) == 0;
-    const long long wh   = is_h ? 4096 : 64, wlw = is_h ? 64 : 1;
+    const long long wh   = is_h ? 256 : 16, wlw = is_h ? 16 : 1;
     for (int it = warp >> 2; it < g * NMB; it += NQ) {
       const int wl = it / NMB, mb = it % NMB;
       const int a  = 8 * (r >> 4) + (r & 7) + 64 * mb; // this row's frame
@@ -443,7 +426,7 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
           for (int c = 0; c < 8; ++c) {
             // columns 16 half + c (h of frame b) and 16 half + 8 + c (l of frame b)
             const int b = 16 * cb + 8 * half + c + 64 * mb;
-            long long e = wh * (long long)(int)v[16 * half + c] + wlw * (long long)(int)v[16 * half + 8 + c];
+            long long e = wh * (long long)v[16 * half + c] + wlw * (long long)v[16 * half + 8 + c];
             e += __shfl_xor_sync(0xFFFFFFFFu, e, 8);
             if (is_h && a <= b && (M == 128 || lane < 16))
               atomicAdd(&aw[b], (unsigned long long)e);
@@ -459,25 +442,14 @@ __global__ void __launch_bounds__(GroupCov<FMT, T, NG, HOP8>::NTHR, GroupCov<FMT
   }
 }
 
-// int64 accumulator (upper triangle) -> float64 Gram with the shift undone exactly.
-__global__ void cov_i8_finalize_kernel(const unsigned long long *acc, const unsigned long long *sums, int T,
-                                       int64_t P, long long shift, double *gram) {
+// int64 accumulator (upper triangle) -> float64 Gram.
+__global__ void cov_i8_finalize_kernel(const unsigned long long *acc, int T, double *gram) {
   const int w = blockIdx.y;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= T * T)
     return;
-  const int       i = e / T, j = e % T;
-  const long long g = (long long)acc[(int64_t)w * T * T + min(i, j) * T + max(i, j)] +
-                      shift * (long long)(sums[(int64_t)w * T + i] + sums[(int64_t)w * T + j]) -
-                      shift * shift * (long long)P;
-  gram[(int64_t)w * T * T + e] = (double)g;
-}
-
-int launch_i8_finalize(const unsigned long long *acc, const unsigned long long *sums, int T, int64_t P,
-                       long long shift, int nwin, double *gram, cudaStream_t s) {
-  cov_i8_finalize_kernel<<<dim3((T * T + 255) / 256, nwin), 256, 0, s>>>(acc, sums, T, P, shift, gram);
-  note_launch();
-  return launch_status("cov_i8_finalize_kernel");
+  const int i = e / T, j = e % T;
+  gram[(int64_t)w * T * T + e] = (double)acc[(int64_t)w * T * T + min(i, j) * T + max(i, j)];
 }
 
 template <int T>
@@ -508,23 +480,26 @@ int launch_tc_group(const FrameRing &ring, int64_t P, int nwin, void *ws, double
   using G               = GroupCov<FMT, T, NG, HOP8>;
   const int     ngroups = (nwin + NG - 1) / NG;
   const int64_t ntiles  = (P + kTcPX - 1) / kTcPX;
-  // at most ~256K pixels per CTA keeps every int32 accumulator entry below 63*63*256K < 2^31
-  const int64_t min_ctas = (P + (1 << 18) - 1) >> 18;
-  // one wave: the CTAs of all groups fit the SMs at once, the SMs split evenly between the groups
-  const int ctas = (int)std::max<int64_t>(
-      min_ctas, std::min<int64_t>(std::max<int64_t>(1, (int64_t)G::PER_SM * sm_count() / ngroups), ntiles));
+  // the CTAs of all groups fit the SMs at once, the SMs split evenly between the groups: one wave, or as
+  // many full ones as keep a CTA at 512 tiles (65536 pixels, the accumulators' range)
+  const int64_t min_ctas = (ntiles + 511) / 512, slots = (int64_t)G::PER_SM * sm_count();
+  int64_t       waves    = 1;
+  while (waves * slots / ngroups < min_ctas)
+    ++waves;
+  const int ctas = (int)std::max<int64_t>(min_ctas, std::min<int64_t>(std::max<int64_t>(1, waves * slots / ngroups), ntiles));
   uint32_t ncols = 32; // a power of two
   while (ncols < (uint32_t)(G::WCOL * std::min(nwin, NG)))
     ncols *= 2;
-  auto *acc  = reinterpret_cast<unsigned long long *>(ws);
-  auto *sums = acc + (size_t)nwin * T * T;
-  HF_CUDA(cudaMemsetAsync(acc, 0, ((size_t)nwin * T * T + (size_t)nwin * T) * sizeof(unsigned long long), s));
+  auto *acc = reinterpret_cast<unsigned long long *>(ws);
+  HF_CUDA(cudaMemsetAsync(acc, 0, (size_t)nwin * T * T * sizeof(unsigned long long), s));
   auto kern = cov_tc_group_kernel<FMT, T, NG, HOP8>;
   HF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem));
-  kern<<<dim3(ctas, ngroups), G::NTHR, G::smem, s>>>(ring, P, nwin, ncols, acc, sums, status);
+  kern<<<dim3(ctas, ngroups), G::NTHR, G::smem, s>>>(ring, P, nwin, ncols, acc, status);
   note_launch();
   HF_TRY(launch_status("cov_tc_group_kernel"));
-  return launch_i8_finalize(acc, sums, T, P, FMT == HF_U8 ? 128 : 2048, nwin, gram, s);
+  cov_i8_finalize_kernel<<<dim3((T * T + 255) / 256, nwin), 256, 0, s>>>(acc, T, gram);
+  note_launch();
+  return launch_status("cov_i8_finalize_kernel");
 }
 
 // T = 64 windows that overlap on an 8-frame grid stage each frame once per group of four; the other
@@ -552,7 +527,7 @@ size_t cov_tc_workspace_bytes(int T, int64_t P, int nwin) {
   const int64_t ntiles = (P + kTcPX - 1) / kTcPX;
   const int64_t ctas   = std::max<int64_t>(1, std::min<int64_t>((3LL * sm_count() + nwin - 1) / nwin, ntiles));
   const size_t f16 = (size_t)(nwin * ctas) * T * T * sizeof(float) + (size_t)(nwin * ctas) * T * sizeof(double) + 256;
-  const size_t i8  = ((size_t)nwin * T * T + (size_t)nwin * T) * sizeof(unsigned long long) + 256;
+  const size_t i8  = (size_t)nwin * T * T * sizeof(unsigned long long) + 256;
   return std::max(f16, i8);
 }
 

@@ -37,6 +37,28 @@ def test_integer_gram_is_exact(cuda, T, fmt, hop, nwin, H, W, form):
     assert p.status() == 0
 
 
+@pytest.mark.parametrize("W", [256, 257 * 2])  # 512 tiles in one CTA; a few more: two CTAs per window
+def test_integer_gram_accumulator_range(cuda, W):
+    """As many windows as the GPU has SMs and full-scale samples: the largest sums a CTA accumulates."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    T, hop, H = 128, 8, 256 if W == 256 else 128
+    nwin = torch.cuda.get_device_properties(0).multi_processor_count
+    n, P = T + hop * (nwin - 1), H * W
+    ring = torch.full((n * P * 3 // 2,), 255, dtype=torch.uint8, device=cuda)
+    ring[7 * P * 3 // 2:8 * P * 3 // 2] = 0  # frame 7 of the first window
+    p = pl.Pipeline(pl.PipelineConfig(height=H, width=W, frames=T, hop=hop, z_begin=1, z_end=2, input_dtype=hf.HF_MONO12P,
+                                      propagation=hf.HF_PROP_NONE, clutter_rank=1, max_batch=nwin, form=1))
+    p.run(ring, n, 0, nwin)
+    for w in (0, 1, nwin - 1):
+        gram, _ = p.inspect(w)
+        exp = np.full((T, T), float(P * 4095 * 4095))
+        if w == 0:
+            exp[7, :] = exp[:, 7] = 0.0
+        assert np.array_equal(gram.cpu().numpy(), exp), w
+
+
 def _check_pairs(a, ev, V, r):
     n = a.shape[0]
     scale = np.abs(a).max()
