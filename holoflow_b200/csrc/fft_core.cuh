@@ -304,4 +304,28 @@ __device__ __forceinline__ void four_step_b_sw(float2 *y, int k1, const float2 *
   dft_reg<32, INV>(y);
 }
 
+__device__ __noinline__ static float hypot_call(float x, float y) { return hypotf(x, y); }
+
+// |y| of 32 values in place (into .x), without overflow or underflow of the squares: hypotf for all of
+// them when any square leaves its safe range.  One test for the 32: a test per value, with its own
+// branch, kept the square roots from overlapping (544 us against 398 us for the row moments of 112 planes of 1024^2).
+__device__ __forceinline__ void abs32(float2 (&y)[32]) {
+  float lo = 1.f, hi = 1.f, sq[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    sq[i] = fmaf(y[i].x, y[i].x, y[i].y * y[i].y);
+    lo    = fminf(lo, sq[i]);
+    hi    = fmaxf(hi, sq[i]);
+  }
+  if (lo >= 1e-30f && hi <= 1e37f) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      y[i].x = __fsqrt_rn(sq[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      y[i].x = hypot_call(y[i].x, y[i].y);
+  }
+}
+
 } // namespace hf

@@ -474,6 +474,8 @@ int launch_col_pass(const ColPass &pass, int mode, const MomentSpec *mom, int nw
       return launch_col_tf(a, nwin, s);
     HF_CHECK_ARG(a.row_lo == 0 && a.row_hi == a.H, "transfer-function columns: zero rows need the strip kernel");
   }
+  if ((mode == COL_COMPLEX || mode == COL_MAGNITUDE) && col_strip_supported(a))
+    return launch_col_strip(a, mode == COL_MAGNITUDE, nwin, s);
   if (fft_fast_length(a.H)) {
     if (a.inverse) {
       HF_DISPATCH_N1(a.H, return (launch_col_fast<N1, true>(a, mode, m, nwin, s)))

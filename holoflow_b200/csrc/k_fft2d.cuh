@@ -72,6 +72,8 @@ bool row_ring_supported(const RowPass &a);
 int  launch_row_ring(const RowPass &a, int nwin, cudaStream_t s);
 bool row_moments_ring_supported(const ColPass &a);
 int  launch_row_moments_ring(const ColPass &a, const MomentSpec &m, int nwin, cudaStream_t s);
+bool col_strip_supported(const ColPass &a);
+int  launch_col_strip(const ColPass &a, bool magnitude, int nwin, cudaStream_t s);
 bool col_tf_supported(const ColPass &a);
 int  launch_col_tf(const ColPass &a, int nwin, cudaStream_t s);
 int  launch_row_any(const RowPass &a, int nwin, cudaStream_t s);

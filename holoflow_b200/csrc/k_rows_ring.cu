@@ -119,30 +119,6 @@ __global__ void __launch_bounds__(32 * ring_warps<N1>(false), 1) row_ring_kernel
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-__device__ __noinline__ float hypot_call(float x, float y) { return hypotf(x, y); }
-
-// |y| of 32 values in place (into .x), without overflow or underflow of the squares: hypotf for all of
-// them when any square leaves its safe range.  One test for the 32: a test per value, with its own
-// branch, kept the square roots from overlapping (544 us against 398 us, see above).
-__device__ __forceinline__ void abs32(float2 (&y)[32]) {
-  float lo = 1.f, hi = 1.f, sq[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    sq[i] = fmaf(y[i].x, y[i].x, y[i].y * y[i].y);
-    lo    = fminf(lo, sq[i]);
-    hi    = fmaxf(hi, sq[i]);
-  }
-  if (lo >= 1e-30f && hi <= 1e37f) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      y[i].x = __fsqrt_rn(sq[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      y[i].x = hypot_call(y[i].x, y[i].y);
-  }
-}
-
 // A warp owns one image row of a window for every plane and keeps the three sums of its 32 outputs
 // per lane in registers (they were read, added to and written back in shared memory per plane).
 template <int N1, bool INV>

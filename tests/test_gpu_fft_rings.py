@@ -115,3 +115,28 @@ def test_short_column_moments(cuda, H, W, nwin, nz, shift, mask, form):
         exp = O.reconstruct_window(x[w * T:(w + 1) * T].astype(np.float64), cfg)
         for i, m in enumerate([m for m in range(3) if mask >> m & 1]):
             assert O.rel_l2(got[w, i], exp[m]) < (1e-3 if form else 1e-4), (w, m)
+
+
+@pytest.mark.parametrize("H", [64, 128, 256, 512, 768, 1024])
+@pytest.mark.parametrize("B", [1, 2, 17])
+@pytest.mark.parametrize("mag,skip", [(True, True), (False, True), (False, False)])
+def test_fresnel_column_strips(cuda, H, B, mag, skip):
+    """Groups of planes in the column strips: one, full groups, a remainder; strided outputs; zeros and
+    magnitudes whose squares leave float32's range."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    W = 64
+    rng = np.random.default_rng(H + B)
+    x = _complex(rng, (B, H, W))
+    exp = O.fresnel(x, LAM, DX, DX, 0.2, output_magnitude=mag, skip_phase_shift=skip)
+    plan = pl.FresnelPlan(B, H, W, hf.HF_CF32, LAM, DX, 0.2, output_magnitude=mag, skip_phase_shift=skip)
+    dev = torch.from_numpy(x).to(cuda)
+    tol = 2e-6 * math.log2(H * W)  # the bound of the other Fresnel tests
+    assert O.rel_l2(plan(dev).cpu().numpy(), exp) < tol
+    out = torch.empty((H, W, B), dtype=torch.float32 if mag else torch.complex64, device=cuda).permute(2, 0, 1)
+    assert O.rel_l2(plan(dev, out).cpu().numpy(), exp) < tol
+    if mag:
+        for scale in (1e-24, 1e30):
+            assert O.rel_l2(plan(dev * scale).cpu().numpy().astype(np.float64) / scale, exp) < tol
+        assert float(plan(dev * 0.0).abs().max()) == 0.0
