@@ -3,11 +3,11 @@
 // work buffers fit in shared memory; the direct O(n^2) sums of k_fft2d.cu remain for the rest.
 //
 // Bound: the direct sums evaluated a sine and a cosine per product, 25.8 ms of rows and 15.3 ms of
-// columns for 2 windows x 10 planes of 600 x 800; both passes here take 0.2 ms together (0.31 GB
-// of planes read and written: shared-memory and barrier bound at about 1.5 TB/s).  A CTA here transforms R rows (or a strip of C
-// columns) in shared memory with the staged FFT of fft_any.cuh, so a pass reads and writes each
-// plane once; the CTAs are persistent over the row groups (strips), so the twiddle table w_n^e is
-// built once per CTA.
+// columns for 2 windows x 10 planes of 600 x 800; the passes here take 91 and 83 us (0.31 GB of planes
+// read and written, 1.8 TB/s: shared-memory and barrier bound).  A CTA transforms R rows (or a strip of
+// C columns) in shared memory with the staged FFT of fft_any.cuh, so a pass reads and writes each plane
+// once; the CTAs are persistent over the row groups (strips), so the twiddle table w_n^e is built once
+// per CTA.  The rows stay one after the other: interleaved as the columns are, they took 94 us (91).
 #include <algorithm>
 
 #include "fft_any.cuh"
@@ -20,7 +20,7 @@ constexpr int    kAnyThreads = 256;
 constexpr int    kAnyMaxN    = 8192;
 constexpr int    kAnyRB      = 4;          // rows per thread of a dense stage
 constexpr int    kAnyMaxRows = 16;
-constexpr size_t kAnySmem    = 104 * 1024; // two CTAs per SM
+constexpr size_t kAnySmem    = 112 * 1024; // two CTAs per SM
 constexpr size_t kAnySmemMax = 220 * 1024; // one CTA per SM (long transforms)
 
 // w_n^e for e < n.  The angle is reduced to a quadrant q and a fraction r / n of it in exact
@@ -77,14 +77,14 @@ __global__ void __launch_bounds__(kAnyThreads, 2) any_rows_kernel(const __grid_c
       for (int u = 0; u < U; ++u) {
         const int t = t0 + u * kAnyThreads;
         if (t < rows * n)
-          b0[t] = a.pre != nullptr ? cmul(v[u], L[u]) : v[u];
+          b0[t] = flip(a.pre != nullptr ? cmul(v[u], L[u]) : v[u], a.inverse != 0);
       }
     }
     __syncthreads();
-    const float2 *res = fft_rows_smem<kAnyRB>(b0, b1, n, rows, pl, tw, a.inverse != 0);
+    const float2 *res = fft_smem<kAnyRB>(b0, b1, row_layout(n, rows), pl, tw);
     for (int t = threadIdx.x; t < rows * n; t += blockDim.x) {
       const int r = fdiv(t, pl.by_n), i = t - r * n;
-      a.out[s_out[r] + i] = res[t];
+      a.out[s_out[r] + i] = flip(res[t], a.inverse != 0);
     }
   }
 }
@@ -95,13 +95,13 @@ __device__ __forceinline__ float any_abs(float2 v) {
   return s >= 1e-30f && s <= 1e37f ? __fsqrt_rn(s) : hypotf(v.x, v.y);
 }
 
-// A strip of C (a power of two) columns of one plane, transposed into rows of pitch n | 1.
+// A strip of C (a power of two) columns of one plane, interleaved in shared memory as they lie in it.
 __global__ void __launch_bounds__(kAnyThreads, 2) any_cols_kernel(const __grid_constant__ ColPass a,
-                                                               const __grid_constant__ GPlan pl, int C, int nstrip,
+                                                               const __grid_constant__ GPlan pl, FastDiv by_C, int nstrip,
                                                                int64_t nwork, int magnitude) {
   extern __shared__ __align__(16) float2 sm[];
-  const int n = pl.n, P = n | 1, Cp = (C + kAnyRB - 1) / kAnyRB * kAnyRB, lc = 31 - __clz(C);
-  float2   *tw = sm, *b0 = sm + n, *b1 = b0 + (size_t)Cp * P;
+  const int n = pl.n, C = (int)by_C.d, lc = 31 - __clz(C);
+  float2   *tw = sm, *b0 = sm + n, *b1 = b0 + (size_t)C * n;
   any_twiddles(tw, n);
   for (int64_t wk = blockIdx.x; wk < nwork; wk += gridDim.x) {
     const int64_t img = wk / nstrip;
@@ -119,19 +119,19 @@ __global__ void __launch_bounds__(kAnyThreads, 2) any_cols_kernel(const __grid_c
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int t = t0 + u * kAnyThreads, y = t >> lc, c = t & (C - 1);
+        const int t = t0 + u * kAnyThreads;
         if (t < n * C)
-          b0[c * P + y] = v[u];
+          b0[t] = flip(v[u], a.inverse != 0);
       }
     }
     __syncthreads();
-    const float2 *res = fft_rows_smem<kAnyRB>(b0, b1, P, C, pl, tw, a.inverse != 0);
+    const float2 *res = fft_smem<kAnyRB>(b0, b1, strip_layout(by_C), pl, tw);
     const int64_t o0  = w * a.out_win + plane * a.out_plane;
     for (int t = threadIdx.x; t < n * C; t += blockDim.x) {
       const int y = t >> lc, c = t & (C - 1);
       if (c >= cw)
         continue;
-      const float2  v = res[c * P + y];
+      const float2  v = flip(res[t], a.inverse != 0);
       const int64_t o = o0 + (int64_t)y * a.out_row + (int64_t)(x0 + c) * a.out_col;
       if (magnitude)
         reinterpret_cast<float *>(a.out)[o] = any_abs(v);
@@ -164,9 +164,10 @@ int launch_row_any(const RowPass &a, int nwin, cudaStream_t s) {
   GPlan pl;
   if (!make_plan(a.N, pl, kAnyMaxN))
     return fail(HF_ERR_UNSUPPORTED, "row pass: no plan for this length");
-  int R = kAnyMaxRows; // the most rows (a multiple of kAnyRB) that leave two CTAs per SM
+  int R = kAnyMaxRows; // at most as many rows as leave two CTAs per SM
   while (R > kAnyRB && any_smem(a.N, R, a.N) > kAnySmem)
     R -= kAnyRB;
+  R = plan_rows(pl, 1, R, kAnyThreads);
   const int64_t nrows = (int64_t)nwin * a.nplanes * a.H;
   const size_t  smem  = any_smem(a.N, R, a.N);
   unsigned      grid  = 0;
@@ -181,14 +182,14 @@ int launch_col_any(const ColPass &a, int magnitude, int nwin, cudaStream_t s) {
   if (!make_plan(a.H, pl, kAnyMaxN))
     return fail(HF_ERR_UNSUPPORTED, "column pass: no plan for this length");
   int C = 16; // at least 4 columns, so that a row of the strip is a whole 32-byte sector
-  while (C > kAnyRB && any_smem(a.H, C, a.H | 1) > kAnySmem)
+  while (C > kAnyRB && any_smem(a.H, C, a.H) > kAnySmem)
     C /= 2;
   const int     nstrip = (a.W + C - 1) / C;
   const int64_t nwork  = (int64_t)nwin * a.nplanes * nstrip;
-  const size_t  smem   = any_smem(a.H, C, a.H | 1);
+  const size_t  smem   = any_smem(a.H, C, a.H);
   unsigned      grid   = 0;
   HF_TRY(any_grid(any_cols_kernel, smem, nwork, &grid));
-  any_cols_kernel<<<grid, kAnyThreads, smem, s>>>(a, pl, C, nstrip, nwork, magnitude);
+  any_cols_kernel<<<grid, kAnyThreads, smem, s>>>(a, pl, make_div((uint32_t)C), nstrip, nwork, magnitude);
   note_launch();
   return launch_status("any_cols_kernel");
 }

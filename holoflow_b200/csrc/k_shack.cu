@@ -13,11 +13,11 @@
 //    (window gather x input lens for the short-time Fresnel transform; mean removal and cosine
 //    taper inside the correlation ROI; normalised cross power against the reference spectrum),
 //    transformed in shared memory and stored contiguously.
-//  - shk_cols_kernel<MODE>: a strip of C columns of one image, transposed into shared memory,
+//  - shk_cols_kernel<MODE>: a strip of C columns of one image, interleaved in shared memory,
 //    transformed along the height, with the post-operation of MODE (complex, |.|, or real part x
 //    scale).
-//  - shk_cols_mean_kernel: the same for the mean of |.| over the band planes, kMeanPlanes planes'
-//    strips per transform, the next group's strips arriving by cp.async into a third buffer while
+//  - shk_cols_mean_kernel: the same for the mean of |.| over the band planes, up to kMeanPlanes
+//    planes' strips per transform, the next group's strips arriving by cp.async into a third buffer while
 //    the current group is transformed, and the per-sub-aperture fftshift fused into the store.
 //  - shk_roi_mean_kernel, shk_peak_kernel (first maximum + parabolic refinement, one CTA per map),
 //    shk_slopes_kernel (one thread) and shk_zfit_kernel (one warp): the reference's float32 sequences,
@@ -41,7 +41,7 @@ constexpr int kShkMaxN     = 1024; // longest transform side
 constexpr int kShkThreads  = 256;
 constexpr int kRedThreads  = 1024; // one CTA per correlation map for the ROI mean and the peak
 constexpr int kShkMaxRows  = 16;   // rows per CTA of the row pass
-constexpr int kMeanPlanes  = 4;    // planes per transform in the band-mean column pass
+constexpr int kMeanPlanes  = 4;    // most planes per transform in the band-mean column pass
 constexpr int kShkMaxModes = 9; // Noll 2..10
 
 std::vector<float2> twiddle_table(int n) {
@@ -59,7 +59,11 @@ struct DevPlan {
   int     n   = 0;
   GPlan  *pl  = nullptr;
   float2 *tw  = nullptr;
+  int     R   = 1; // rows per CTA of the row pass along this length
+  int     G   = 1; // planes per transform of the band-mean column pass
 };
+
+int mean_strip(int h) { return std::max(1, (h <= 256 ? 16 : (h <= 512 ? 8 : 4)) / kMeanPlanes); }
 
 void release(DevPlan &d) {
   cudaFree(d.pl), cudaFree(d.tw);
@@ -70,7 +74,9 @@ int dev_plan_init(DevPlan &d, int n) {
   GPlan pl;
   if (!make_plan(n, pl, kShkMaxN))
     return fail(HF_ERR_UNSUPPORTED, "autofocus: transform sides must be in 2..1024");
-  d.n                         = n;
+  d.n = n;
+  d.R = plan_rows(pl, 1, std::max(1, std::min(kShkMaxRows, 4096 / n)), kShkThreads);
+  d.G = plan_rows(pl, mean_strip(n), kMeanPlanes * mean_strip(n), kShkThreads) / mean_strip(n);
   const std::vector<float2> t = twiddle_table(n);
   HF_TRY(cuda_status(cudaMalloc(&d.pl, sizeof(GPlan)), "autofocus: plan"));
   HF_TRY(cuda_status(cudaMalloc(&d.tw, t.size() * sizeof(float2)), "autofocus: twiddles"));
@@ -204,13 +210,13 @@ template <int MODE> __global__ void __launch_bounds__(kShkThreads, 4) shk_rows_k
         const float  mag = sqrtf(p.x * p.x + p.y * p.y);
         v                = mag <= 1e-12f ? make_float2(0.f, 0.f) : make_float2(p.x / mag, p.y / mag);
       }
-      b0[t] = v;
+      b0[t] = flip(v, a.inv);
     }
   }
   __syncthreads();
-  const float2 *res = fft_rows_smem<1>(b0, b1, n, rows, spl, tw, a.inv);
+  const float2 *res = fft_smem<1>(b0, b1, row_layout(n, rows), spl, tw);
   for (int t = threadIdx.x; t < rows * n; t += blockDim.x)
-    a.out[row0 * n + t] = res[t];
+    a.out[row0 * n + t] = flip(res[t], a.inv);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -222,7 +228,7 @@ struct ColArgs {
   const GPlan  *pl; // device copy of the transform plan along the column
   int           h;  // column length
   const float2 *tw; // [h]
-  int           C, pitch, nstrip, w;
+  int           C, nstrip, w;
   bool          inv;
   const float2 *in;   // [images][h][w]
   float2       *outc; // COL_COMPLEX (may equal in)
@@ -231,8 +237,9 @@ struct ColArgs {
   int           planes;  // COL_MEAN_MAG: planes averaged; image = plane * nwin + window
   int64_t       nwin;
   int           shift;   // COL_MEAN_MAG: fftshift of every image on store
+  int           G;       // COL_MEAN_MAG: planes per transform
   float         scale;   // COL_REAL
-  FastDiv       by_hc;   // h C (plane index of a strip element)
+  FastDiv       by_cols; // interleaved columns: C, or G C
 };
 
 // One image's strip (COL_COMPLEX, COL_MAG, COL_REAL): loads, transform, post-operation.
@@ -240,8 +247,8 @@ template <int MODE> __global__ void __launch_bounds__(kShkThreads, 3) shk_cols_k
   static_assert(MODE != COL_MEAN_MAG, "the band mean runs in shk_cols_mean_kernel");
   extern __shared__ __align__(16) float2 sm[];
   __shared__ GPlan spl;
-  const int h = a.h, C = a.C, P = a.pitch;
-  float2   *tw = sm, *b0 = sm + h, *b1 = b0 + (size_t)C * P;
+  const int h = a.h, C = a.C;
+  float2   *tw = sm, *b0 = sm + h, *b1 = b0 + (size_t)C * h;
   for (int e = threadIdx.x; e < h; e += blockDim.x)
     tw[e] = a.tw[e];
   for (int i = threadIdx.x; i < (int)(sizeof(GPlan) / 4); i += blockDim.x)
@@ -266,17 +273,16 @@ template <int MODE> __global__ void __launch_bounds__(kShkThreads, 3) shk_cols_k
       const int t = t0 + u * blockDim.x;
       if (t >= h * C)
         break;
-      const int y = t >> lc, c = t & (C - 1);
-      b0[c * P + y] = ld[u];
+      b0[t] = flip(ld[u], a.inv);
     }
   }
   __syncthreads();
-  const float2 *res = fft_rows_smem<1>(b0, b1, P, C, spl, tw, a.inv);
+  const float2 *res = fft_smem<1>(b0, b1, strip_layout(a.by_cols), spl, tw);
   for (int t = threadIdx.x; t < h * C; t += blockDim.x) {
     const int y = t >> lc, c = t & (C - 1);
     if (c >= cw)
       continue;
-    const float2  v = res[c * P + y];
+    const float2  v = flip(res[t], a.inv);
     const int64_t o = (img * h + y) * (int64_t)a.w + x0 + c;
     if constexpr (MODE == COL_COMPLEX)
       a.outc[o] = a.post ? cmul(v, a.post[(int64_t)y * a.w + x0 + c]) : v;
@@ -294,17 +300,24 @@ __device__ __forceinline__ void cp_async8(float2 *dst, const float2 *src, bool o
                : "memory");
 }
 
-// The band-mean column pass (COL_MEAN_MAG) with its loads overlapped: each group of kMeanPlanes
-// planes' strips arrives by cp.async into a third buffer while the previous group is transformed
-// and accumulated.  |.| = sqrtf(x^2 + y^2) summed in band order in float32, then divided by the
-// plane count.
-__global__ void __launch_bounds__(kShkThreads, 2) shk_cols_mean_kernel(ColArgs a) {
+__device__ __forceinline__ void cp_async16(float2 *dst, const float2 *src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(ok ? 16 : 0)
+               : "memory");
+}
+
+// The band-mean column pass (COL_MEAN_MAG) with its loads overlapped: each group of G planes' strips
+// arrives by cp.async into a third buffer while the previous group is transformed and accumulated
+// (forward transforms only).  |.| = sqrtf(x^2 + y^2) summed in band order in float32, then divided by
+// the plane count.  The strips keep the image's order in shared memory, so a copy takes 16 bytes and no
+// stage has bank conflicts: transposed into rows, 8 bytes a copy, a window of 28 planes x 25 sub-apertures
+// of 204 x 204 took 277 us (233 MB read), here 185.
+__global__ void __launch_bounds__(kShkThreads, 3) shk_cols_mean_kernel(ColArgs a) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ GPlan spl;
-  constexpr int G  = kMeanPlanes;
-  const int     h = a.h, C = a.C, P = a.pitch;
-  float2       *tw = sm, *bx = sm + h, *b1 = bx + (size_t)G * C * P, *by = b1 + (size_t)G * C * P;
-  float        *acc = reinterpret_cast<float *>(by + (size_t)G * C * P); // [h * C]
+  const int     G = a.G, h = a.h, C = a.C, S = G * C; // S columns interleaved: column g C + c
+  float2       *tw = sm, *bx = sm + (h + 1) / 2 * 2, *b1 = bx + (size_t)S * h, *by = b1 + (size_t)S * h;
+  float        *acc = reinterpret_cast<float *>(by + (size_t)S * h); // [h * C]
   for (int e = threadIdx.x; e < h; e += blockDim.x)
     tw[e] = a.tw[e];
   for (int i = threadIdx.x; i < (int)(sizeof(GPlan) / 4); i += blockDim.x)
@@ -315,14 +328,23 @@ __global__ void __launch_bounds__(kShkThreads, 2) shk_cols_mean_kernel(ColArgs a
   const int     lc = 31 - __clz(C); // C is a power of two
   for (int t = threadIdx.x; t < h * C; t += blockDim.x)
     acc[t] = 0.f;
-  // the strip of plane g of a group sits at rows [g C, g C + C) of a buffer, transposed
+  // the strip of plane g of a group: columns [g C, g C + C) of a buffer, in pieces of 16 bytes where the
+  // image rows are aligned to them
+  const bool pairs = C % 2 == 0 && a.w % 2 == 0 && (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
+  const int  unit = pairs ? 2 : 1, per = C / unit, lp = 31 - __clz(per);
   const auto issue = [&](int pl, float2 *dst) {
     const int ng = min(G, a.planes - pl);
-    for (int t = threadIdx.x; t < ng * h * C; t += blockDim.x) {
-      const int     g = fdiv(t, a.by_hc), r = t - g * h * C, y = r >> lc, c = r & (C - 1);
-      const int64_t src = (int64_t)(pl + g) * a.nwin + img;
-      const bool    ok  = c < cw;
-      cp_async8(dst + (g * C + c) * P + y, a.in + (src * h + y) * (int64_t)a.w + x0 + (ok ? c : 0), ok);
+    for (int g = 0; g < ng; ++g) {
+      const float2 *src = a.in + (((int64_t)(pl + g) * a.nwin + img) * h) * a.w + x0;
+      float2       *d   = dst + g * C;
+      for (int t = threadIdx.x; t < h * per; t += blockDim.x) {
+        const int  y = t >> lp, c = (t & (per - 1)) * unit;
+        const bool ok = c < cw; // cw is even where pairs are copied
+        if (pairs)
+          cp_async16(d + y * S + c, src + y * a.w + (ok ? c : 0), ok);
+        else
+          cp_async8(d + y * S + c, src + y * a.w + (ok ? c : 0), ok);
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -334,17 +356,17 @@ __global__ void __launch_bounds__(kShkThreads, 2) shk_cols_mean_kernel(ColArgs a
     __syncthreads(); // every thread's copies of this group have landed
     if (pl + G < a.planes)
       issue(pl + G, spare); // the next group streams in during this group's transforms
-    const float2 *res = fft_rows_smem<1>(cur, b1, P, ng * C, spl, tw, a.inv);
+    const float2 *res = fft_smem<1>(cur, b1, strip_layout(a.by_cols), spl, tw);
     for (int t = threadIdx.x; t < h * C; t += blockDim.x) {
       const int y = t >> lc, c = t & (C - 1);
       if (c >= cw)
         continue;
-      const float2 v = res[c * P + y];
+      const float2 v = res[y * S + c];
       float        s = acc[t] + sqrtf(v.x * v.x + v.y * v.y); // band order, float32
 #pragma unroll
-      for (int g = 1; g < G; ++g)
+      for (int g = 1; g < kMeanPlanes; ++g)
         if (g < ng) {
-          const float2 u = res[(g * C + c) * P + y];
+          const float2 u = res[y * S + g * C + c];
           s += sqrtf(u.x * u.x + u.y * u.y);
         }
       acc[t] = s;
@@ -366,21 +388,14 @@ __global__ void __launch_bounds__(kShkThreads, 2) shk_cols_mean_kernel(ColArgs a
 }
 
 size_t rows_smem(int n, int R) { return (size_t)n * sizeof(float2) * (1 + 2 * (size_t)R); }
-int    rows_per_cta(int n) { return std::max(1, std::min(kShkMaxRows, 4096 / n)); }
-int    col_strip(int h, bool mean) {
-  const int c = h <= 256 ? 16 : (h <= 512 ? 8 : 4);
-  return mean ? std::max(1, c / kMeanPlanes) : c; // the mean pass holds kMeanPlanes planes' strips
-}
-size_t cols_smem(int h, int C, bool mean) {
-  const int P = h | 1; // odd pitch: the transposed loads spread over the banks
-  const int G = mean ? kMeanPlanes : 1;
-  // the band-mean pass holds a third buffer for the group in flight
-  return (size_t)h * sizeof(float2) + (mean ? 3 : 2) * (size_t)G * C * P * sizeof(float2) +
-         (mean ? (size_t)h * C * sizeof(float) : 0);
+int    col_strip(int h) { return h <= 256 ? 16 : (h <= 512 ? 8 : 4); }
+// G: planes of the band-mean pass, which holds a third buffer for the group in flight (0: one image)
+size_t cols_smem(int h, int C, int G) {
+  return (size_t)(h + 1) / 2 * 2 * sizeof(float2) + (G > 0 ? 3 * (size_t)G : 2) * C * h * sizeof(float2) +
+         (G > 0 ? (size_t)h * C * sizeof(float) : 0);
 }
 
 template <int MODE> int launch_rows(RowArgs a, cudaStream_t s) {
-  a.R             = rows_per_cta(a.n);
   const size_t sm = rows_smem(a.n, a.R);
   HF_CUDA(cudaFuncSetAttribute(shk_rows_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int64_t grid = (a.n_rows + a.R - 1) / a.R;
@@ -392,11 +407,10 @@ template <int MODE> int launch_rows(RowArgs a, cudaStream_t s) {
 }
 
 template <int MODE> int launch_cols(ColArgs a, int64_t images, cudaStream_t s) {
-  a.C             = col_strip(a.h, MODE == COL_MEAN_MAG);
-  a.pitch         = a.h | 1;
+  a.C             = MODE == COL_MEAN_MAG ? mean_strip(a.h) : col_strip(a.h);
   a.nstrip        = (a.w + a.C - 1) / a.C;
-  a.by_hc         = make_div((uint32_t)(a.h * a.C));
-  const size_t sm = cols_smem(a.h, a.C, MODE == COL_MEAN_MAG);
+  a.by_cols       = make_div((uint32_t)(MODE == COL_MEAN_MAG ? a.G * a.C : a.C));
+  const size_t sm = cols_smem(a.h, a.C, MODE == COL_MEAN_MAG ? a.G : 0);
   const int64_t grid = images * a.nstrip;
   if (grid > INT_MAX)
     return fail(HF_ERR_UNSUPPORTED, "short-time Fresnel: too many column strips");
@@ -1047,12 +1061,12 @@ int hf_stfd_exec(hf_stfd *f, const void *in, void *out, hf_stream_t s) {
   const int64_t nwin = (int64_t)f->nwy * f->nwx;
   float2       *rows = f->output == HF_STFD_COMPLEX ? static_cast<float2 *>(out) : f->scratch;
   RowArgs       ra{};
-  ra.pl = f->pw.pl, ra.n = f->pw.n, ra.tw = f->pw.tw, ra.n_rows = f->planes * nwin * f->win_h, ra.inv = false, ra.out = rows;
+  ra.pl = f->pw.pl, ra.R = f->pw.R, ra.n = f->pw.n, ra.tw = f->pw.tw, ra.n_rows = f->planes * nwin * f->win_h, ra.inv = false, ra.out = rows;
   ra.field = in, ra.real_in = f->real_in, ra.H = f->H, ra.W = f->W, ra.win_h = f->win_h, ra.nwx = f->nwx;
   ra.nwy = f->nwy, ra.stride_y = f->sy, ra.stride_x = f->sx, ra.global_lens = f->global, ra.lens = f->lens;
   HF_TRY(launch_rows<ROW_STFD>(ra, s));
   ColArgs ca{};
-  ca.pl = f->ph.pl, ca.h = f->ph.n, ca.tw = f->ph.tw, ca.w = f->win_w, ca.inv = false, ca.in = rows;
+  ca.pl = f->ph.pl, ca.G = f->ph.G, ca.h = f->ph.n, ca.tw = f->ph.tw, ca.w = f->win_w, ca.inv = false, ca.in = rows;
   switch (f->output) {
   case HF_STFD_COMPLEX:
     ca.outc = static_cast<float2 *>(out), ca.post = f->wlens;
@@ -1269,11 +1283,11 @@ int hf_shslopes_exec(hf_shslopes *p, const float *images, float *slopes, float *
   HF_TRY(launch_status("shk_roi_mean_kernel"));
   // forward transform of the prepared images: rows (mean removal + taper fused), then columns
   RowArgs ra{};
-  ra.pl = p->pw.pl, ra.n = p->pw.n, ra.tw = p->pw.tw, ra.n_rows = rows, ra.inv = false, ra.out = p->spec;
+  ra.pl = p->pw.pl, ra.R = p->pw.R, ra.n = p->pw.n, ra.tw = p->pw.tw, ra.n_rows = rows, ra.inv = false, ra.out = p->spec;
   ra.img = images, ra.means = p->means, ra.taper = p->taper, ra.h = p->h;
   HF_TRY(launch_rows<ROW_XPACK>(ra, s));
   ColArgs ca{};
-  ca.pl = p->ph.pl, ca.h = p->ph.n, ca.tw = p->ph.tw, ca.w = p->w, ca.inv = false, ca.in = p->spec, ca.outc = p->spec;
+  ca.pl = p->ph.pl, ca.G = p->ph.G, ca.h = p->ph.n, ca.tw = p->ph.tw, ca.w = p->w, ca.inv = false, ca.in = p->spec, ca.outc = p->spec;
   HF_TRY(launch_cols<COL_COMPLEX>(ca, p->count, s));
   if (p->mode == 1) { // FullPairwise: every pair of active samples, pair_batch maps at a time
     HF_CHECK_ARG(maps == nullptr, "ShackHartmannSlopes: FullPairwise correlation-map output is not supported");
@@ -1281,12 +1295,12 @@ int hf_shslopes_exec(hf_shslopes *p, const float *images, float *slopes, float *
     for (int64_t e0 = 0; e0 < p->npairs; e0 += p->pair_batch) {
       const int nb = (int)std::min<int64_t>(p->pair_batch, p->npairs - e0);
       RowArgs   rp{};
-      rp.pl = p->pw.pl, rp.n = p->pw.n, rp.tw = p->pw.tw, rp.n_rows = (int64_t)nb * p->h, rp.inv = true;
+      rp.pl = p->pw.pl, rp.R = p->pw.R, rp.n = p->pw.n, rp.tw = p->pw.tw, rp.n_rows = (int64_t)nb * p->h, rp.inv = true;
       rp.out = p->pcross, rp.spec = p->spec, rp.h = p->h, rp.pair_src = p->pair_src, rp.pair_dst = p->pair_dst;
       rp.pair0 = e0;
       HF_TRY(launch_rows<ROW_PAIR>(rp, s));
       ColArgs cp{};
-      cp.pl = p->ph.pl, cp.h = p->ph.n, cp.tw = p->ph.tw, cp.w = p->w, cp.inv = true, cp.in = p->pcross, cp.outf = p->pmaps;
+      cp.pl = p->ph.pl, cp.G = p->ph.G, cp.h = p->ph.n, cp.tw = p->ph.tw, cp.w = p->w, cp.inv = true, cp.in = p->pcross, cp.outf = p->pmaps;
       cp.scale = (float)(1.0 / ((double)p->h * p->w)); // inverse_fft_scale
       HF_TRY(launch_cols<COL_REAL>(cp, nb, s));
       shk_peak_kernel<<<nb, kRedThreads, 0, s>>>(p->pmaps, p->pshift, p->h, p->w);
@@ -1302,11 +1316,11 @@ int hf_shslopes_exec(hf_shslopes *p, const float *images, float *slopes, float *
   }
   // cross power against the centre spectrum (fused into the inverse row pass), inverse columns
   RowArgs rb{};
-  rb.pl = p->pw.pl, rb.n = p->pw.n, rb.tw = p->pw.tw, rb.n_rows = rows, rb.inv = true, rb.out = p->cross;
+  rb.pl = p->pw.pl, rb.R = p->pw.R, rb.n = p->pw.n, rb.tw = p->pw.tw, rb.n_rows = rows, rb.inv = true, rb.out = p->cross;
   rb.spec = p->spec, rb.ref_img = p->center, rb.h = p->h;
   HF_TRY(launch_rows<ROW_CROSS>(rb, s));
   ColArgs cb{};
-  cb.pl = p->ph.pl, cb.h = p->ph.n, cb.tw = p->ph.tw, cb.w = p->w, cb.inv = true, cb.in = p->cross, cb.outf = mo;
+  cb.pl = p->ph.pl, cb.G = p->ph.G, cb.h = p->ph.n, cb.tw = p->ph.tw, cb.w = p->w, cb.inv = true, cb.in = p->cross, cb.outf = mo;
   cb.scale = (float)(1.0 / ((double)p->h * p->w)); // backward norm (cross_correlation2.cu:119-125)
   HF_TRY(launch_cols<COL_REAL>(cb, p->count, s));
   shk_peak_kernel<<<p->count, kRedThreads, 0, s>>>(mo, p->shifts, p->h, p->w);

@@ -12,6 +12,7 @@ import math
 import pathlib
 
 SIZES = [4, 8, 16, 24, 32, 48, 64]
+ROOTS = [3, 5, 6, 7, 8, 9, 10, 11, 12, 13, 15, 16, 17]  # radices of the any-length transform: c_rootP
 
 
 def fmt(v: float) -> str:
@@ -51,6 +52,9 @@ def main(out: pathlib.Path) -> None:
             else:
                 tvals.append("{%s, %s}" % (fmt(s), fmt(c / s)))
         lines.append("static __constant__ float2 c_twt%d[%d] = {%s};" % (n, n, ", ".join(tvals)))
+    for n in ROOTS:
+        vals = ["{%s, %s}" % (fmt(math.cos(2.0 * math.pi * k / n)), fmt(-math.sin(2.0 * math.pi * k / n))) for k in range(n)]
+        lines.append("static __constant__ float2 c_root%d[%d] = {%s};" % (n, n, ", ".join(vals)))
     text = "\n".join(lines) + "\n"
     if not out.exists() or out.read_text() != text:  # keep the mtime (and the build) when unchanged
         out.write_text(text)

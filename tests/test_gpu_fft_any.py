@@ -84,3 +84,20 @@ def test_overflowing_squares_keep_their_magnitude(cuda):
         plan = pl.FresnelPlan(1, 5, 7, hf.HF_CF32, LAM, DX, 0.3, output_magnitude=True)
         got = plan(torch.from_numpy(x).to(cuda)).cpu().numpy()
         np.testing.assert_allclose(got, np.full((1, 5, 7), scale), rtol=1e-5)
+
+
+@pytest.mark.parametrize("h,w", [(2, 2), (3, 3), (16, 7), (23, 24), (34, 51), (204, 12), (255, 9), (300, 10), (607, 3),
+                                 (1024, 2)])
+@pytest.mark.parametrize("nz", [1, 3, 4, 5, 9])
+def test_band_mean_columns(cuda, h, w, nz):
+    """The sub-aperture band mean: plane groups with and without a remainder, odd and even widths (copies
+    of one and two samples), strips wider than the image, columns with a dense stage."""
+    import torch
+    from holoflow_b200 import autofocus as af
+    from oracle import shack as SH
+    rng = np.random.default_rng(h + w + nz)
+    x = (rng.standard_normal((nz, 2 * h, 2 * w)) + 1j * rng.standard_normal((nz, 2 * h, 2 * w))).astype(np.complex64)
+    op = af.ShortTimeFresnel(x.shape, (h, w), (h, w), LAM, DX, DX, 0.25, phase_ref="global", output="mean_magnitude")
+    got = op(torch.from_numpy(x).to(cuda)).cpu().numpy()
+    exp = np.abs(SH.stfd(x, h, w, h, w, LAM, DX, DX, 0.25, "global", False)).mean(axis=0)
+    assert O.rel_l2(got.reshape(exp.shape), exp) < 1e-5  # the bound of the other sub-aperture tests
