@@ -180,7 +180,7 @@ int hf_band_moments(const void *planes, int in_dtype, int nz, int64_t P, const f
     w.w1[k] = freqs[k];
     w.w2[k] = freqs[k] * freqs[k];
   }
-  return launch_band_moments(planes, in_dtype, nz, P, w, moment_mask, out, s);
+  return launch_band_moments(planes, in_dtype, 0, nz, P, w, moment_mask, out, 0, 1, s);
 }
 
 } // extern "C"

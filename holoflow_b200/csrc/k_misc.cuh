@@ -25,8 +25,9 @@ int launch_convert(const void *in, int in_dtype, void *out, int out_dtype, int s
                    void *minmax_ws, cudaStream_t s);
 int launch_mean_axis(const void *in, int in_dtype, int64_t outer, int64_t n, int64_t inner,
                      void *out, bool abs_values, cudaStream_t s);
-int launch_band_moments(const void *planes, int in_dtype, int nz, int64_t P, const MomentWeights &w,
-                        int mask, float *out, cudaStream_t s);
+// Moments of nwin windows of nz planes of P values, in_win values and out_win floats apart.
+int launch_band_moments(const void *planes, int in_dtype, int64_t in_win, int nz, int64_t P, const MomentWeights &w,
+                        int mask, float *out, int64_t out_win, int nwin, cudaStream_t s);
 int launch_fresnel_lens(float2 *lens, int W, int H, float lambda, float z, float dx, cudaStream_t s);
 
 // One value of the Fresnel quadratic-phase lens (fresnel_diffraction.cu:326-341): centred

@@ -315,8 +315,7 @@ static int phase_after_band(hf_plan *p, int nwin, float *out, cudaStream_t s, bo
     memcpy(mw.w1, p->mom.w1, sizeof(mw.w1));
     memcpy(mw.w2, p->mom.w2, sizeof(mw.w2));
     rec = p->timer.begin(s, ST_COLS_MOM);
-    for (int w = 0; w < nwin; ++w)
-      HF_TRY(launch_band_moments(p->band + w * win_px, HF_CF32, p->nz, p->P, mw, d.moment_mask, out + w * owin, s));
+    HF_TRY(launch_band_moments(p->band, HF_CF32, win_px, p->nz, p->P, mw, d.moment_mask, out, owin, nwin, s));
     p->timer.end(s, rec);
     return HF_OK;
   }
@@ -414,8 +413,7 @@ static int phase_after_band(hf_plan *p, int nwin, float *out, cudaStream_t s, bo
       MomentWeights mw;
       memcpy(mw.w1, p->mom.w1, sizeof(mw.w1));
       memcpy(mw.w2, p->mom.w2, sizeof(mw.w2));
-      for (int w = 0; w < nwin; ++w)
-        HF_TRY(launch_band_moments(p->band + w * win_px, HF_CF32, p->nz, p->P, mw, d.moment_mask, out + w * owin, s));
+      HF_TRY(launch_band_moments(p->band, HF_CF32, win_px, p->nz, p->P, mw, d.moment_mask, out, owin, nwin, s));
     }
     p->timer.end(s, rec);
     return zero_leading();

@@ -101,3 +101,24 @@ def test_band_mean_columns(cuda, h, w, nz):
     got = op(torch.from_numpy(x).to(cuda)).cpu().numpy()
     exp = np.abs(SH.stfd(x, h, w, h, w, LAM, DX, DX, 0.25, "global", False)).mean(axis=0)
     assert O.rel_l2(got.reshape(exp.shape), exp) < 1e-5  # the bound of the other sub-aperture tests
+
+
+@pytest.mark.parametrize("nz", [1, 3, 4, 9])
+@pytest.mark.parametrize("prop,H,W", [("none", 7, 18), ("fresnel", 30, 50)])
+def test_moments_of_a_batch(cuda, nz, prop, H, W):
+    """The moment reduction of the general sizes: groups of planes and a remainder, several windows."""
+    import torch
+    import holoflow_b200 as hf
+    from holoflow_b200 import pipeline as pl
+    rng = np.random.default_rng(nz)
+    T, nwin = 20, 3
+    x = rng.integers(0, 4096, (T * nwin, H, W)).astype(np.uint16)
+    p = pl.Pipeline(pl.PipelineConfig(height=H, width=W, frames=T, hop=T, z_begin=1, z_end=1 + nz, input_dtype=hf.HF_U16,
+                                      z=0.3, max_batch=nwin,
+                                      propagation=hf.HF_PROP_NONE if prop == "none" else hf.HF_PROP_FRESNEL))
+    got = p.run(torch.from_numpy(x.view(np.int16)).to(cuda), T * nwin, 0, nwin).cpu().numpy()
+    cfg = O.PathConfig(H, W, T, T, 1, 1 + nz, z=0.3, propagation=prop)
+    for w in range(nwin):
+        exp = O.reconstruct_window(x[w * T:(w + 1) * T].astype(np.float64), cfg)
+        for m in range(3):
+            assert O.rel_l2(got[w, m], exp[m]) < 1e-4, (w, m)
