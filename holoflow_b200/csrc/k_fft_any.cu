@@ -3,8 +3,8 @@
 // work buffers fit in shared memory; the direct O(n^2) sums of k_fft2d.cu remain for the rest.
 //
 // Bound: the direct sums evaluated a sine and a cosine per product, 25.8 ms of rows and 15.3 ms of
-// columns for 2 windows x 10 planes of 600 x 800; the passes here take 91 and 83 us (0.31 GB of planes
-// read and written, 1.8 TB/s: shared-memory and barrier bound).  A CTA transforms R rows (or a strip of
+// columns for 2 windows x 10 planes of 600 x 800; the passes here take 96 and 81 us (0.31 GB of planes
+// read and written, 1.7 TB/s: shared-memory and barrier bound).  A CTA transforms R rows (or a strip of
 // C columns) in shared memory with the staged FFT of fft_any.cuh, so a pass reads and writes each plane
 // once; the CTAs are persistent over the row groups (strips), so the twiddle table w_n^e is built once
 // per CTA.  The rows stay one after the other: interleaved as the columns are, they took 94 us (91).

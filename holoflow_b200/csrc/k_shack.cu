@@ -311,7 +311,7 @@ __device__ __forceinline__ void cp_async16(float2 *dst, const float2 *src, bool 
 // (forward transforms only).  |.| = sqrtf(x^2 + y^2) summed in band order in float32, then divided by
 // the plane count.  The strips keep the image's order in shared memory, so a copy takes 16 bytes and no
 // stage has bank conflicts: transposed into rows, 8 bytes a copy, a window of 28 planes x 25 sub-apertures
-// of 204 x 204 took 277 us (233 MB read), here 185.
+// of 204 x 204 took 277 us (233 MB read), here 178.
 __global__ void __launch_bounds__(kShkThreads, 3) shk_cols_mean_kernel(ColArgs a) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ GPlan spl;
