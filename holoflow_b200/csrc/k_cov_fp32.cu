@@ -13,6 +13,7 @@
 // covers: 165 us).  Measured, 2 windows of 32 x 600 x 800 16-bit frames, kernel + reduction: 331 -> 94 us.
 #include <algorithm>
 
+#include "host/cov_split.hh"
 #include "k_pca.cuh"
 
 namespace hf {
@@ -231,10 +232,9 @@ int launch_reduce(const float *partial, const double *sums, int nblk, int nsum, 
   return launch_status("cov_reduce_kernel");
 }
 
-int cov_ctas(int T, int64_t P, int nwin) {
-  const int64_t ntiles = (P + cov_geom(T).PX - 1) / cov_geom(T).PX;
-  return (int)std::max<int64_t>(1, std::min<int64_t>((2 * sm_count() + nwin - 1) / nwin, ntiles));
-}
+int64_t cov_tiles(int T, int64_t P) { return (P + cov_geom(T).PX - 1) / cov_geom(T).PX; }
+
+int cov_ctas(int T, int64_t P, int nwin) { return (int)cov_split(sm_count(), cov_tiles(T, P), nwin); }
 
 template <int FMT>
 int launch_fmt(const FrameRing &ring, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas, cudaStream_t s) {
@@ -264,8 +264,8 @@ size_t cov_fp32_cta_bytes(int T) {
   return (size_t)g.U * 64 * sizeof(float) + (size_t)T * sizeof(double);
 }
 
-size_t cov_fp32_workspace_bytes(int T, int64_t P, int nwin) {
-  return (size_t)nwin * cov_ctas(T, P, nwin) * cov_fp32_cta_bytes(T) + 256;
+size_t cov_fp32_workspace_bytes(int T, int64_t P, int max_windows) {
+  return (size_t)cov_split_most(sm_count(), cov_tiles(T, P), max_windows) * cov_fp32_cta_bytes(T) + 256;
 }
 
 int launch_cov_fp32(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas,

@@ -355,8 +355,8 @@ __global__ void pca_project_kernel(const float *in, int T, int64_t P, const doub
 
 } // namespace
 
-size_t cov_workspace_bytes(int T, int64_t P, int nwin) {
-  return cov_fp32_supported(T) ? cov_fp32_workspace_bytes(T, P, nwin) : 256;
+size_t cov_workspace_bytes(int T, int64_t P, int max_windows) {
+  return cov_fp32_supported(T) ? cov_fp32_workspace_bytes(T, P, max_windows) : 256;
 }
 
 int launch_covariance(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws,

@@ -18,12 +18,13 @@ struct CovArgs {
   int       nblk;    // CTAs per window (partials per window)
 };
 
-size_t cov_workspace_bytes(int T, int64_t P, int nwin);
+// Workspace of launch_covariance for any call of up to `max_windows` windows.
+size_t cov_workspace_bytes(int T, int64_t P, int max_windows);
 // FP32 CUDA-core Gram matrix, T <= 128, any row alignment (k_cov_fp32.cu); `max_ctas` > 0 caps the CTAs
 // per window, each of which writes cov_fp32_cta_bytes of partials.
 bool   cov_fp32_supported(int T);
 size_t cov_fp32_cta_bytes(int T);
-size_t cov_fp32_workspace_bytes(int T, int64_t P, int nwin);
+size_t cov_fp32_workspace_bytes(int T, int64_t P, int max_windows);
 int    launch_cov_fp32(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram,
                        int max_ctas, cudaStream_t s);
 // Deterministic float64 reduction of block partials; undoes the sample shift exactly.

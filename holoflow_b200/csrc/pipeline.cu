@@ -598,7 +598,7 @@ int hf_plan_create(const hf_desc *desc, hf_plan **out, hf_stream_t stream) {
       // 0.15 ms per 8 windows of 64 x 1024^2); the f16 one of 16-bit samples is the chosen form's
       p->cov_tc = (d.form == HF_FORM_CHOSEN || cov_tc_exact(d.input_dtype)) &&
                   cov_tc_supported(d.input_dtype, T, p->P, p->frame_bytes);
-      size_t wsb = cov_workspace_bytes(T, p->P, (int)B) + cov_workspace_bytes(T, p->P, 1);
+      size_t wsb = cov_workspace_bytes(T, p->P, (int)B); // for every call of 1 .. B windows
       if (p->cov_tc)
         wsb = std::max(wsb, cov_tc_workspace_bytes(T, p->P, (int)B) + cov_tc_workspace_bytes(T, p->P, 1));
       uint8_t *ws = nullptr;
