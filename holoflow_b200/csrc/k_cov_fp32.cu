@@ -1,16 +1,22 @@
-// FP32 Gram matrix of a window's frames on the CUDA cores, any T <= 128, any sample format and any
-// row alignment: 16-bit and float frames, and 8/12-bit frames the tensor-core kernel cannot address.
+// Gram matrix of a window's frames on the CUDA cores, any T <= 128, any sample format and any row
+// alignment: 16-bit and float frames, and 8/12-bit frames the tensor-core kernel cannot address.  Sums in
+// FP32 for the frames that cov_sums_fp32 names (T = 32, 64, 128 in aligned rows), in float64 for the rest,
+// where integer samples give the exact matrix (up to 2^53).
 //
 // Bound: T (T + 1) / 2 products per pixel on the FMA pipe, against shared-memory reads of the
-// operands.  A thread sums an 8 x 8 block of the upper triangle (64 registers): four 16-byte reads
-// feed 64 FMAs, which keeps the two pipes level; the 4 x 4 blocks before read 2 for 16.  The blocks of
-// one pixel occupy U = NB (NB + 1) / 2 threads (NB = ceil(T / 8)) and the CTA's 256 threads work on
-// 256 / U pixels at once.  Samples are staged four frames of one pixel per thread, so the transposed
-// 16-byte stores are conflict-free (row stride = 1 mod 8 chunks), as x - shift, exact in FP32; the
-// shift is undone in float64 from exact integer frame sums (summed from the staged tile: 64-bit shared
-// atomics per sample quad took half of the kernel).
-// Two CTAs of 256 threads per SM (the registers of 288 threads fit once, whose load latency nothing
-// covers: 165 us).  Measured, 2 windows of 32 x 600 x 800 16-bit frames, kernel + reduction: 331 -> 94 us.
+// operands.  A thread sums an 8 x 8 block of the upper triangle: four 16-byte reads feed 64 FMAs, which
+// keeps the two pipes level; the 4 x 4 blocks before read 2 for 16.  The blocks of one pixel occupy
+// U = NB (NB + 1) / 2 threads (NB = ceil(T / 8)) and the CTA's 256 threads work on 256 / U pixels at
+// once.  Samples are staged four frames of one pixel per thread, so the transposed 16-byte stores are
+// conflict-free (row stride = 1 mod 8 chunks).
+//  - FP32: staged as x - shift, exact; the shift is undone in float64 by the reduction, from exact
+//    integer frame sums (summed from the staged tile: 64-bit shared atomics per sample quad took half of
+//    the kernel).  Two CTAs of 256 threads per SM (the registers of 288 threads fit once, whose load
+//    latency nothing covers: 165 us).  Measured, 2 windows of 32 x 600 x 800 16-bit frames, kernel +
+//    reduction: 331 -> 94 us.
+//  - float64: staged as x (exact in FP32) and widened as it is read; the block takes 128 registers, so
+//    one CTA per SM.  Measured, 16 windows of 50 x 16384 16-bit pixels: one thread per entry 2551 us, here
+//    110.
 #include <algorithm>
 
 #include "host/cov_split.hh"
@@ -24,7 +30,7 @@ constexpr int kCovThr = 256;
 
 struct CovGeom {
   int NB, U, G, PX, XS; // 8-frame blocks, upper blocks, pixel groups, pixels per tile, row stride
-  int nxs;              // floats of the tile (and of the final block rows, 8 per thread)
+  int nxs;              // floats of the tile (and of the final block rows, 8 sums per thread)
   size_t smem;
 };
 
@@ -38,7 +44,7 @@ CovGeom cov_geom(int T) {
     if ((size_t)px * g.XS * sizeof(float) <= 48 * 1024 && waste < best - 1e-9)
       best = waste, g.PX = px;
   }
-  g.nxs  = std::max(g.PX * g.XS, 8 * kCovThr);
+  g.nxs  = std::max(g.PX * g.XS, 2 * 8 * kCovThr);
   g.smem = (size_t)g.nxs * sizeof(float) + 128 * (sizeof(int64_t) + sizeof(unsigned long long));
   return g;
 }
@@ -57,9 +63,11 @@ template <int FMT> __device__ __forceinline__ uint32_t raw_sample(const uint8_t 
   }
 }
 
-template <int FMT>
-__global__ void __launch_bounds__(kCovThr, 2) cov_fp32_kernel(FrameRing ring, int T, int64_t P, float shift, CovGeom g,
-                                                              float *partial, double *sums) {
+// Acc: float, or double with shift = 0 and no frame sums.
+template <int FMT, typename Acc>
+__global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
+    cov_cores_kernel(FrameRing ring, int T, int64_t P, float shift, CovGeom g, Acc *partial, double *sums) {
+  constexpr bool kShift = FMT != HF_F32 && sizeof(Acc) == 4;
   extern __shared__ __align__(16) float xs[]; // [PX][XS]
   int64_t            *foff = reinterpret_cast<int64_t *>(xs + g.nxs);                // [128]
   unsigned long long *ssum = reinterpret_cast<unsigned long long *>(foff + 128);     // [128]
@@ -71,12 +79,12 @@ __global__ void __launch_bounds__(kCovThr, 2) cov_fp32_kernel(FrameRing ring, in
     ++bi;
   }
   const int bj = bi + rem;
-  float     acc[8][8];
+  Acc       acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      acc[i][j] = 0.f;
+      acc[i][j] = Acc(0);
   int64_t fsum[4] = {0, 0, 0, 0}; // this warp's share of the sums of frames lane + 32 c
   if (tid < 128) {
     foff[tid] = ring.frame(w, min(tid, T - 1)) - ring.base;
@@ -115,7 +123,7 @@ __global__ void __launch_bounds__(kCovThr, 2) cov_fp32_kernel(FrameRing ring, in
       }
     }
     __syncthreads();
-    if constexpr (FMT != HF_F32) { // frame sums: a tile's (at most 256 values below 2^16) are exact in FP32
+    if constexpr (kShift) { // frame sums: a tile's (at most 256 values below 2^16) are exact in FP32
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int t = (tid & 31) + 32 * c;
@@ -135,49 +143,51 @@ __global__ void __launch_bounds__(kCovThr, 2) cov_fp32_kernel(FrameRing ring, in
       for (int p = grp; p < g.PX; p += g.G) {
         const float4 a0 = *reinterpret_cast<const float4 *>(xa + p * g.XS), a1 = *reinterpret_cast<const float4 *>(xa + p * g.XS + 4);
         const float4 b0 = *reinterpret_cast<const float4 *>(xb + p * g.XS), b1 = *reinterpret_cast<const float4 *>(xb + p * g.XS + 4);
-        const float  va[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float  vb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        const Acc    va[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const Acc    vb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            acc[i][j] = fmaf(va[i], vb[j], acc[i][j]);
+            acc[i][j] = fma(va[i], vb[j], acc[i][j]);
       }
     }
     __syncthreads();
   }
   // the groups' sums of a block row, added in float64 through shared memory (row i of every block at
-  // a time), one float partial per CTA
+  // a time), one partial per CTA
+  Acc *rows = reinterpret_cast<Acc *>(xs);
   const int64_t pidx = ((int64_t)w * gridDim.x + blockIdx.x) * g.U * 64;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     if (grp < g.G)
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        xs[tid * 8 + j] = acc[i][j];
+        rows[tid * 8 + j] = acc[i][j];
     __syncthreads();
     for (int e = tid; e < g.U * 8; e += kCovThr) {
       double s = 0.0;
       for (int q = 0; q < g.G; ++q)
-        s += (double)xs[q * g.U * 8 + e];
-      partial[pidx + (e >> 3) * 64 + 8 * i + (e & 7)] = (float)s;
+        s += (double)rows[q * g.U * 8 + e];
+      partial[pidx + (e >> 3) * 64 + 8 * i + (e & 7)] = (Acc)s;
     }
     __syncthreads();
   }
-  if constexpr (FMT != HF_F32) {
+  if constexpr (kShift) {
 #pragma unroll
     for (int c = 0; c < 4; ++c)
       atomicAdd(&ssum[(tid & 31) + 32 * c], (unsigned long long)fsum[c]);
     __syncthreads();
+    for (int t = tid; t < T; t += kCovThr) // of x - shift
+      sums[((int64_t)w * gridDim.x + blockIdx.x) * T + t] = (double)(long long)ssum[t];
   }
-  for (int t = tid; t < T; t += kCovThr) // of x - shift
-    sums[((int64_t)w * gridDim.x + blockIdx.x) * T + t] = (double)(long long)ssum[t];
 }
 
 // Float64 reduction of the CTA partials in a fixed order (8 interleaved slices per entry, added
 // pairwise); undoes the shift exactly.  `blocked`: partials are the 8 x 8 upper blocks of
-// cov_fp32_kernel, else whole [T][T] matrices of which the upper triangle is read.
-__global__ void __launch_bounds__(256) cov_reduce_kernel(const float *partial, const double *sums, int nblk, int nsum,
+// cov_cores_kernel, else whole [T][T] matrices of which the upper triangle is read.
+template <typename Acc>
+__global__ void __launch_bounds__(256) cov_reduce_kernel(const Acc *partial, const double *sums, int nblk, int nsum,
                                                          int T, int64_t P, double shift, int blocked, double *gram) {
   __shared__ double red[3][8][32];
   const int w = blockIdx.y, lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
@@ -199,7 +209,7 @@ __global__ void __launch_bounds__(256) cov_reduce_kernel(const float *partial, c
   const bool ok = i < T && j < T && i <= j;
   double     s = 0.0, si = 0.0, sj = 0.0;
   if (ok) {
-    const float *pp = partial + (int64_t)w * nblk * per + e;
+    const Acc *pp = partial + (int64_t)w * nblk * per + e;
     for (int b = slice; b < nblk; b += 8)
       s += (double)pp[(int64_t)b * per];
     if (shift != 0.0) {
@@ -224,8 +234,9 @@ __global__ void __launch_bounds__(256) cov_reduce_kernel(const float *partial, c
   gram[(int64_t)w * T * T + j * T + i] = v;
 }
 
-int launch_reduce(const float *partial, const double *sums, int nblk, int nsum, int T, int64_t P, double shift,
-                  int blocked, double *gram, int nwin, cudaStream_t s) {
+template <typename Acc>
+int launch_reduce(const Acc *partial, const double *sums, int nblk, int nsum, int T, int64_t P, double shift, int blocked,
+                  double *gram, int nwin, cudaStream_t s) {
   const int NB = (T + 7) / 8, per = blocked ? NB * (NB + 1) / 2 * 64 : T * T;
   cov_reduce_kernel<<<dim3((per + 31) / 32, nwin), 256, 0, s>>>(partial, sums, nblk, nsum, T, P, shift, blocked, gram);
   note_launch();
@@ -236,41 +247,45 @@ int64_t cov_tiles(int T, int64_t P) { return (P + cov_geom(T).PX - 1) / cov_geom
 
 int cov_ctas(int T, int64_t P, int nwin) { return (int)cov_split(sm_count(), cov_tiles(T, P), nwin); }
 
-template <int FMT>
-int launch_fmt(const FrameRing &ring, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas, cudaStream_t s) {
+template <int FMT, typename Acc>
+int launch_sums(const FrameRing &ring, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas, cudaStream_t s) {
   const CovGeom g     = cov_geom(T);
   const int     ctas  = max_ctas > 0 ? std::min(max_ctas, cov_ctas(T, P, nwin)) : cov_ctas(T, P, nwin);
-  const float   shift = FMT == HF_F32 ? 0.f : (FMT == HF_U8 ? 128.f : 2048.f);
-  auto         *sums  = reinterpret_cast<double *>(ws); // 8-byte aligned first, then the float partials
-  auto         *part  = reinterpret_cast<float *>(sums + (size_t)nwin * ctas * T);
-  HF_CUDA(cudaFuncSetAttribute(cov_fp32_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
-  cov_fp32_kernel<FMT><<<dim3(ctas, nwin), kCovThr, g.smem, s>>>(ring, T, P, shift, g, part, sums);
+  const float   shift = FMT == HF_F32 || sizeof(Acc) == 8 ? 0.f : (FMT == HF_U8 ? 128.f : 2048.f);
+  auto         *sums  = reinterpret_cast<double *>(ws); // 8-byte aligned first, then the partials
+  auto         *part  = reinterpret_cast<Acc *>(sums + (sizeof(Acc) == 8 ? 0 : (size_t)nwin * ctas * T));
+  auto          kern  = cov_cores_kernel<FMT, Acc>;
+  HF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+  kern<<<dim3(ctas, nwin), kCovThr, g.smem, s>>>(ring, T, P, shift, g, part, sums);
   note_launch();
-  HF_TRY(launch_status("cov_fp32_kernel"));
-  return launch_reduce(part, sums, ctas, ctas, T, P, (double)shift, 1, gram, nwin, s);
+  HF_TRY(launch_status("cov_cores_kernel"));
+  return launch_reduce<Acc>(part, sums, ctas, ctas, T, P, (double)shift, 1, gram, nwin, s);
+}
+
+template <int FMT>
+int launch_fmt(const FrameRing &ring, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas, cudaStream_t s) {
+  return cov_sums_fp32(ring, T, P) ? launch_sums<FMT, float>(ring, T, P, nwin, ws, gram, max_ctas, s)
+                                   : launch_sums<FMT, double>(ring, T, P, nwin, ws, gram, max_ctas, s);
 }
 
 } // namespace
 
 int launch_cov_finalize(const float *partial, const double *sums, int nblk, int nsum, int T, int64_t P, double shift,
                         double *gram, int nwin, cudaStream_t s) {
-  return launch_reduce(partial, sums, nblk, nsum, T, P, shift, 0, gram, nwin, s);
+  return launch_reduce<float>(partial, sums, nblk, nsum, T, P, shift, 0, gram, nwin, s);
 }
 
-bool cov_fp32_supported(int T) { return T >= 1 && T <= 128; }
+bool cov_cores_supported(int T) { return T >= 1 && T <= 128; }
 
-size_t cov_fp32_cta_bytes(int T) {
-  const CovGeom g = cov_geom(T);
-  return (size_t)g.U * 64 * sizeof(float) + (size_t)T * sizeof(double);
+size_t cov_cores_workspace_bytes(int T, int64_t P, int max_windows) {
+  // float64 partials of the blocks; FP32 ones with the T frame sums take less
+  const size_t cta = (size_t)cov_geom(T).U * 64 * sizeof(double);
+  return (size_t)cov_split_most(sm_count(), cov_tiles(T, P), max_windows) * cta + 256;
 }
 
-size_t cov_fp32_workspace_bytes(int T, int64_t P, int max_windows) {
-  return (size_t)cov_split_most(sm_count(), cov_tiles(T, P), max_windows) * cov_fp32_cta_bytes(T) + 256;
-}
-
-int launch_cov_fp32(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas,
-                    cudaStream_t s) {
-  HF_CHECK_ARG(cov_fp32_supported(T), "covariance: at most 128 frames");
+int launch_cov_cores(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram, int max_ctas,
+                     cudaStream_t s) {
+  HF_CHECK_ARG(cov_cores_supported(T), "covariance: at most 128 frames");
   switch (fmt) {
   case HF_MONO12P: return launch_fmt<HF_MONO12P>(ring, T, P, nwin, ws, gram, max_ctas, s);
   case HF_U16: return launch_fmt<HF_U16>(ring, T, P, nwin, ws, gram, max_ctas, s);

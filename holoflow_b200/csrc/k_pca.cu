@@ -16,8 +16,8 @@ namespace hf {
 
 namespace {
 
-// Any T, no workspace (more than 128 frames, or callers without one): one thread per upper entry,
-// float64 accumulation, no shift.
+// Any T, no workspace (more than 128 frames, or callers that have or may use none): one thread per upper
+// entry, float64 accumulation, no shift.
 template <int FMT>
 __global__ void cov_generic_kernel(FrameRing ring, int T, int64_t P, double *gram) {
   const int w = blockIdx.y;
@@ -356,14 +356,14 @@ __global__ void pca_project_kernel(const float *in, int T, int64_t P, const doub
 } // namespace
 
 size_t cov_workspace_bytes(int T, int64_t P, int max_windows) {
-  return cov_fp32_supported(T) ? cov_fp32_workspace_bytes(T, P, max_windows) : 256;
+  return cov_cores_supported(T) ? cov_cores_workspace_bytes(T, P, max_windows) : 256;
 }
 
 int launch_covariance(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws,
                       double *gram, cudaStream_t s) {
   HF_CHECK_ARG(T > 0 && P > 0 && nwin > 0, "covariance: empty problem");
-  if (ws != nullptr && cov_fp32_supported(T))
-    return launch_cov_fp32(ring, fmt, T, P, nwin, ws, gram, 0, s);
+  if (ws != nullptr && cov_cores_supported(T))
+    return launch_cov_cores(ring, fmt, T, P, nwin, ws, gram, 0, s);
   return launch_cov_direct(ring, fmt, T, P, nwin, gram, s);
 }
 
@@ -440,34 +440,29 @@ int scratch_address(void **ptr) {
   return HF_OK;
 }
 
-// One CTA's partials as the batch limit counts them.  T = 32, 64 and 128 on 4-byte-aligned rows keep
-// the documented T*T*4*G + T*8 bytes (the kernel needs no more); the others, which have no limit, count
-// what the kernel writes and take the direct kernel beyond it.
-size_t fixed_cta_bytes(int T, bool limited) {
+// One CTA's partials as the batch limit counts them (the kernel needs no more).
+size_t fixed_cta_bytes(int T) {
   const int G = T == 32 ? 4 : (T == 64 ? 2 : 1);
-  return limited ? (size_t)G * T * T * sizeof(float) + (size_t)T * sizeof(double) : cov_fp32_cta_bytes(T);
+  return (size_t)G * T * T * sizeof(float) + (size_t)T * sizeof(double);
 }
 } // namespace
 
 int launch_covariance_fixed_scratch(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, double *gram,
                                     cudaStream_t s) {
   HF_CHECK_ARG(T > 0 && P > 0 && nwin > 0, "covariance: empty problem");
-  const bool limited = (T == 32 || T == 64 || T == 128) && P % 8 == 0 && ring.frame_bytes % 4 == 0 &&
-                       (reinterpret_cast<uintptr_t>(ring.base) & 3) == 0;
-  const size_t usable = HF_COVARIANCE_NOALLOC_SCRATCH_BYTES - 256;
-  const size_t fit    = cov_fp32_supported(T) ? usable / ((size_t)nwin * fixed_cta_bytes(T, limited)) : 0;
-  if (fit < 1) {
-    if (!limited)
-      return launch_cov_direct(ring, fmt, T, P, nwin, gram, s);
+  // only the FP32 sums use the workspace, which calls that overlap in time would share
+  if (!cov_sums_fp32(ring, T, P))
+    return launch_cov_direct(ring, fmt, T, P, nwin, gram, s);
+  const size_t fit = (HF_COVARIANCE_NOALLOC_SCRATCH_BYTES - 256) / ((size_t)nwin * fixed_cta_bytes(T));
+  if (fit < 1)
     return fail(HF_ERR_INVALID,
                 "hf_covariance_noalloc: batch " + std::to_string(nwin) + " at T = " + std::to_string(T) +
                     " needs more than the fixed " +
                     std::to_string(HF_COVARIANCE_NOALLOC_SCRATCH_BYTES >> 20) +
                     " MiB workspace; split the batch or use hf_covariance with a workspace");
-  }
   void *ws = nullptr;
   HF_TRY(scratch_address(&ws));
-  return launch_cov_fp32(ring, fmt, T, P, nwin, ws, gram, (int)std::min<size_t>(fit, (size_t)1 << 20), s);
+  return launch_cov_cores(ring, fmt, T, P, nwin, ws, gram, (int)std::min<size_t>(fit, (size_t)1 << 20), s);
 }
 
 } // namespace hf

@@ -20,13 +20,18 @@ struct CovArgs {
 
 // Workspace of launch_covariance for any call of up to `max_windows` windows.
 size_t cov_workspace_bytes(int T, int64_t P, int max_windows);
-// FP32 CUDA-core Gram matrix, T <= 128, any row alignment (k_cov_fp32.cu); `max_ctas` > 0 caps the CTAs
-// per window, each of which writes cov_fp32_cta_bytes of partials.
-bool   cov_fp32_supported(int T);
-size_t cov_fp32_cta_bytes(int T);
-size_t cov_fp32_workspace_bytes(int T, int64_t P, int max_windows);
-int    launch_cov_fp32(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram,
-                       int max_ctas, cudaStream_t s);
+// Frames whose Gram matrix is summed in FP32 (x - shift, FP32 partials per CTA): T = 32, 64, 128 in whole
+// groups of 8 pixels and 4-byte-aligned rows.  The others are summed in float64.
+inline bool cov_sums_fp32(const FrameRing &ring, int T, int64_t P) {
+  return (T == 32 || T == 64 || T == 128) && P % 8 == 0 && ring.frame_bytes % 4 == 0 &&
+         (reinterpret_cast<uintptr_t>(ring.base) & 3) == 0;
+}
+// CUDA-core Gram matrix, T <= 128, any row alignment (k_cov_fp32.cu); `max_ctas` > 0 caps the CTAs per
+// window, each of which writes at most T*T*4*G + T*8 bytes of FP32 partials (G = 4, 2, 1 for T = 32, 64, 128).
+bool   cov_cores_supported(int T);
+size_t cov_cores_workspace_bytes(int T, int64_t P, int max_windows);
+int    launch_cov_cores(const FrameRing &ring, int fmt, int T, int64_t P, int nwin, void *ws, double *gram,
+                        int max_ctas, cudaStream_t s);
 // Deterministic float64 reduction of block partials; undoes the sample shift exactly.
 int launch_cov_finalize(const float *partial, const double *sums, int nblk, int nsum, int T, int64_t P,
                         double shift, double *gram, int nwin, cudaStream_t s);

@@ -92,8 +92,12 @@ int hf_temporal_dft(const void *in, int in_dtype, int64_t batch, int T, int64_t 
 /* ---- a8: PCA / SVD clutter filter (PcaTask, holotask/src/syncs/pca.cc:68-119) -------------
  * hf_covariance: gram[b] = X_b^T X_b (T x T, float64, row-major, symmetric), X_b = [T][P] frames
  * of in_dtype (HF_U8, HF_U16, HF_MONO12P, HF_F32).  No centring, no 1/N (pca.cc:92-98).
- * `ws` must hold hf_covariance_workspace_bytes(T, P) bytes per batch item (it may be NULL when
- * `in` is not 4-byte aligned: such input takes the direct kernel, which needs no workspace). */
+ * T = 32, 64, 128 with P % 8 == 0, 4-byte-aligned frames and a 4-byte-aligned `in` are summed in FP32
+ * (of x - shift, undone exactly; one FP32 partial per CTA), every other input in float64 (exact for
+ * integer samples up to 2^53).
+ * `ws` must hold hf_covariance_workspace_bytes(T, P) bytes per batch item.  It may be NULL for the
+ * inputs summed in float64: these then take the direct kernel (one thread per entry, no workspace), as
+ * T > 128 does always. */
 size_t hf_covariance_workspace_bytes(int T, int64_t P);
 int    hf_covariance(const void *in, int in_dtype, int64_t batch, int T, int64_t P, double *gram,
                      void *ws, hf_stream_t s);
@@ -110,11 +114,12 @@ int    hf_covariance(const void *in, int in_dtype, int64_t batch, int T, int64_t
  *    and caches it; make that first call before any stream capture on that device.  The cached
  *    address belongs to the device's primary context: after cudaDeviceReset on that device it is
  *    stale, so a process that resets a device must not call this function on it again.
- *  - `in` may have any alignment: a base that is not 4-byte aligned takes the direct kernel.
- *  - A batch whose partial sums cannot fit (batch x one CTA's partials, T*T*4*G + T*8 bytes with
+ *  - `in` may have any alignment.  The inputs that hf_covariance sums in float64 take the direct kernel
+ *    here, which uses no workspace: the limits below are not for them, and their calls may overlap.
+ *  - Otherwise a batch whose partial sums cannot fit (batch x one CTA's partials, T*T*4*G + T*8 bytes with
  *    G = 4, 2, 1 for T = 32, 64, 128) is rejected with HF_ERR_INVALID; larger problems are split
  *    over fewer CTAs so that they fit, which can change the float32 rounding of the partials.
- *  - Calls on one device share the array: calls whose work can overlap in time (different
+ *  - Calls on one device share the array: calls that use it and whose work can overlap in time (different
  *    streams without ordering, or different host threads) race; serialise them on one stream.
  * Arguments, results and errors are otherwise those of hf_covariance. */
 #define HF_COVARIANCE_NOALLOC_SCRATCH_BYTES (16u << 20)
