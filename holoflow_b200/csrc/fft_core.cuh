@@ -307,20 +307,33 @@ __device__ __forceinline__ void four_step_b_sw(float2 *y, int k1, const float2 *
 __device__ __noinline__ static float hypot_call(float x, float y) { return hypotf(x, y); }
 
 // |y| of 32 values in place (into .x), without overflow or underflow of the squares: hypotf for all of
-// them when any square leaves its safe range.  One test for the 32: a test per value, with its own
-// branch, kept the square roots from overlapping (544 us against 398 us for the row moments of 112 planes of 1024^2).
+// them when any square leaves its safe range or is not a number.  One test for the 32: a test per value,
+// with its own branch, kept the square roots from overlapping (544 us against 398 us for the row moments
+// of 112 planes of 1024^2).  Zeros (blank regions) are no reason for hypotf, but the square root leaves its
+// fast path for them, so values with zeros among them take its root of the range's low end instead:
+// those moments of zero planes take 389 us (others 381), 545 with hypotf and 444 with the square roots of zeros.
 __device__ __forceinline__ void abs32(float2 (&y)[32]) {
-  float lo = 1.f, hi = 1.f, sq[32];
+  // as integers the non-negative floats are in order, and infinities and NaN beyond them
+  constexpr float kLo = 1e-30f, kHi = 1e37f;
+  const uint32_t  range = __float_as_uint(kHi) - __float_as_uint(kLo);
+  uint32_t        off = 0u; // the largest distance from kLo; below it they wrap, a zero stands next to kHi
+  float           sq[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     sq[i] = fmaf(y[i].x, y[i].x, y[i].y * y[i].y);
-    lo    = fminf(lo, sq[i]);
-    hi    = fmaxf(hi, sq[i]);
+    const bool zero = ((__float_as_uint(y[i].x) | __float_as_uint(y[i].y)) & 0x7FFFFFFFu) == 0u;
+    off = max(off, zero ? range + 1u : __float_as_uint(sq[i]) - __float_as_uint(kLo));
   }
-  if (lo >= 1e-30f && hi <= 1e37f) {
+  if (off <= range) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
       y[i].x = __fsqrt_rn(sq[i]);
+  } else if (off == range + 1u) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const float r = __fsqrt_rn(fmaxf(sq[i], kLo));
+      y[i].x        = sq[i] == 0.f ? 0.f : r;
+    }
   } else {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
