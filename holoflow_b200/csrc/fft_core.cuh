@@ -306,29 +306,39 @@ __device__ __forceinline__ void four_step_b_sw(float2 *y, int k1, const float2 *
 
 __device__ __noinline__ static float hypot_call(float x, float y) { return hypotf(x, y); }
 
+__device__ __forceinline__ float max_nan(float a, float b) { // NaN if either is
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // |y| of 32 values in place (into .x), without overflow or underflow of the squares: hypotf for all of
 // them when any square leaves its safe range or is not a number.  One test for the 32: a test per value,
 // with its own branch, kept the square roots from overlapping (544 us against 398 us for the row moments
 // of 112 planes of 1024^2).  Zeros (blank regions) are no reason for hypotf, but the square root leaves its
 // fast path for them, so values with zeros among them take its root of the range's low end instead:
-// those moments of zero planes take 389 us (others 381), 545 with hypotf and 444 with the square roots of zeros.
+// those moments of zero planes take 414 us (others 383), 545 with hypotf and 444 with the square roots of zeros.
 __device__ __forceinline__ void abs32(float2 (&y)[32]) {
-  // as integers the non-negative floats are in order, and infinities and NaN beyond them
   constexpr float kLo = 1e-30f, kHi = 1e37f;
-  const uint32_t  range = __float_as_uint(kHi) - __float_as_uint(kLo);
-  uint32_t        off = 0u; // the largest distance from kLo; below it they wrap, a zero stands next to kHi
-  float           sq[32];
+  float           lo = 1.f, hi = 1.f, sq[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     sq[i] = fmaf(y[i].x, y[i].x, y[i].y * y[i].y);
-    const bool zero = ((__float_as_uint(y[i].x) | __float_as_uint(y[i].y)) & 0x7FFFFFFFu) == 0u;
-    off = max(off, zero ? range + 1u : __float_as_uint(sq[i]) - __float_as_uint(kLo));
+    lo    = fminf(lo, sq[i]);
+    hi    = max_nan(hi, sq[i]);
   }
-  if (off <= range) {
+  bool fast = lo >= kLo && hi <= kHi;
+  if (fast) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
       y[i].x = __fsqrt_rn(sq[i]);
-  } else if (off == range + 1u) {
+    return;
+  }
+  fast = hi <= kHi;
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    fast = fast && (sq[i] >= kLo || (y[i].x == 0.f && y[i].y == 0.f));
+  if (fast) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const float r = __fsqrt_rn(fmaxf(sq[i], kLo));

@@ -10,7 +10,7 @@
 // cp.async groups is waited for.  Rows run plane by plane at one image row, so the warps of a CTA
 // read the same lens row.  8 windows x 28 planes of 1024^2 with the lens: 753 -> 637 us (5.9 TB/s); 4
 // windows x 56 planes of 1024 x 1536: 1430 -> 1161 us; 4 windows x 28 planes of 768^2 placed in 1024^2:
-// 1240 -> 221 us; inverse rows and moments of those: 487 -> 381 us.
+// 1240 -> 221 us; inverse rows and moments of those: 487 -> 383 us.
 #include <algorithm>
 
 #include "fft_core.cuh"
