@@ -21,18 +21,17 @@
 //    1.4e-7.
 //  - 128 threads per CTA, three CTAs per SM (about 170 registers each): 128 / KG lanes x 4 pixels by
 //    KG bin groups.  The CTAs are persistent over the pixel tiles of a window, so W is staged once,
-//    and the next tile's samples stream in by cp.async while this one is summed.
+//    and the next tile's samples stream in by cp.async while this one is summed (long windows, whose two
+//    tiles do not fit beside W, hold one).
 #include <algorithm>
 
 #include "frames.cuh"
+#include "host/band_geom.hh"
 #include "k_band.cuh"
 
 namespace hf {
 
 namespace {
-
-constexpr int kBandPX  = 4;   // pixels per thread
-constexpr int kBandThr = 128;
 
 template <int FMT> struct FmtBytes;
 template <> struct FmtBytes<HF_MONO12P> { static constexpr int num = 3, den = 2; };
@@ -110,15 +109,15 @@ __device__ __forceinline__ void stage_tile(uint8_t *dst, const uint8_t *base, co
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-template <int FMT, int NB>
+template <int FMT, int NB, int STAGES>
 __global__ void __launch_bounds__(kBandThr, 3) band_dft_fp32_kernel(BandArgs a, int KG, int nzpad, int unit, int vec) {
   extern __shared__ __align__(16) uint8_t smem[];
   constexpr int  num = FmtBytes<FMT>::num, den = FmtBytes<FMT>::den;
   constexpr bool kLevel = FMT != HF_F32;
   const int     w       = blockIdx.y;
   const int     tile_px = kBandThr * kBandPX / KG, bytes = tile_px * num / den;
-  uint8_t *stage = smem;                                                        // [2][T][bytes]
-  float2  *w_sh  = reinterpret_cast<float2 *>(smem + 2 * (size_t)a.T * bytes);  // [T][nzpad]
+  uint8_t *stage = smem;                                                            // [STAGES][T][bytes]
+  float2  *w_sh  = reinterpret_cast<float2 *>(smem + STAGES * (size_t)a.T * bytes); // [T][nzpad]
   float2  *wsum  = w_sh + (size_t)a.T * nzpad;                                  // [nzpad] sum_t W
   int64_t *foff  = reinterpret_cast<int64_t *>(wsum + nzpad);                    // [T] frame offsets
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -151,9 +150,13 @@ __global__ void __launch_bounds__(kBandThr, 3) band_dft_fp32_kernel(BandArgs a, 
 
   const int kgi = warp % KG, g = (warp / KG) * 32 + lane; // bin group, 4-pixel group of the tile
   int       s   = 0;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, s ^= 1) {
-    fetch(tile + gridDim.x, s ^ 1);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, s ^= STAGES - 1) {
+    if constexpr (STAGES == 2) {
+      fetch(tile + gridDim.x, s ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    }
     __syncthreads();
     const uint8_t *rows = stage + (size_t)s * a.T * bytes;
     const int64_t  p0   = tile * tile_px + (int64_t)g * kBandPX;
@@ -226,7 +229,9 @@ __global__ void __launch_bounds__(kBandThr, 3) band_dft_fp32_kernel(BandArgs a, 
         }
       }
     }
-    __syncthreads(); // this tile's rows are read: the stage takes the tile after next
+    __syncthreads(); // this tile's rows are read: the stage takes the tile after next (one stage: the next)
+    if constexpr (STAGES == 1)
+      fetch(tile + gridDim.x, 0);
   }
 }
 
@@ -266,40 +271,21 @@ template <int FMT> __global__ void band_dft_simple_kernel(BandArgs a) {
   }
 }
 
-// Bins per thread (even, at most 14), bin groups side by side, and shared memory of a launch.
-struct BandGeom {
-  int    NB, KG, nzpad;
-  size_t smem;
-};
-
-template <int FMT> BandGeom band_geom(int T, int nz) {
-  const int k  = (nz + 13) / 14; // bin groups
-  BandGeom  g{};
-  g.NB = std::max(4, ((nz + k - 1) / k + 1) / 2 * 2);
-  // the fewest groups side by side (the largest tile) that leave three CTAs per SM, else the most
-  for (g.KG = 1;; g.KG *= 2) {
-    g.nzpad = (nz + g.KG * g.NB - 1) / (g.KG * g.NB) * g.KG * g.NB;
-    g.smem  = 2 * (size_t)T * (kBandThr * kBandPX / g.KG) * FmtBytes<FMT>::num / FmtBytes<FMT>::den +
-             (size_t)(T + 1) * g.nzpad * sizeof(float2) + (size_t)T * sizeof(int64_t);
-    if (g.KG == 4 || g.smem <= 74 * 1024)
-      return g;
-  }
-}
-
 template <int FMT, int NB> int launch_nb(const BandArgs &a, const BandGeom &g, int unit, int vec, int nwin, cudaStream_t s) {
-  HF_CUDA(cudaFuncSetAttribute(band_dft_fp32_kernel<FMT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+  auto kern = g.stages == 2 ? band_dft_fp32_kernel<FMT, NB, 2> : band_dft_fp32_kernel<FMT, NB, 1>;
+  HF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
   const int     tile_px = kBandThr * kBandPX / g.KG;
   const int64_t ntiles  = (a.P + tile_px - 1) / tile_px;
-  const int     per_sm  = std::max(1, std::min(3, (int)(220 * 1024 / g.smem)));
+  const int     per_sm  = std::max(1, std::min(3, (int)(kBandSmem / g.smem)));
   const int64_t ctas    = std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)per_sm * sm_count() / nwin));
-  band_dft_fp32_kernel<FMT, NB><<<dim3((unsigned)ctas, nwin), kBandThr, g.smem, s>>>(a, g.KG, g.nzpad, unit, vec);
+  kern<<<dim3((unsigned)ctas, nwin), kBandThr, g.smem, s>>>(a, g.KG, g.nzpad, unit, vec);
   note_launch();
   return launch_status("band_dft_fp32_kernel");
 }
 
 template <int FMT> int launch_fp32(const BandArgs &a, int nwin, cudaStream_t s) {
-  const BandGeom g = band_geom<FMT>(a.T, a.nz);
-  if (g.smem > 220 * 1024)
+  const BandGeom g = band_geom(a.T, a.nz, FmtBytes<FMT>::num, FmtBytes<FMT>::den);
+  if (g.smem > kBandSmem)
     return HF_ERR_UNSUPPORTED;
   const uintptr_t rows = reinterpret_cast<uintptr_t>(a.ring.base) | (uintptr_t)a.ring.frame_bytes;
   const int       unit = rows % 16 == 0 ? 16 : (rows % 4 == 0 ? 4 : 1);
