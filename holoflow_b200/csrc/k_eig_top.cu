@@ -125,8 +125,8 @@ __device__ __forceinline__ double reciprocal(double x) {
   return fabs(x) > 1e-30 && fabs(x) < 1e30 ? rcp_seeded(x, rcp_approx((float)x)) : 1.0 / x;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 1) eig_top_kernel(const double *a_in, double *evecs, double *evals, int *info,
+template <int NT, int PER_SM>
+__global__ void __launch_bounds__(NT, PER_SM) eig_top_kernel(const double *a_in, double *evecs, double *evals, int *info,
                                                         int n, int r) {
   constexpr int kWarps = NT / 32;
   constexpr int RM     = NT / 4;          // rows the CTA can hold
@@ -648,7 +648,12 @@ int launch_eig_top(const double *a, double *evecs, double *evals, int *info, int
   HF_CHECK_ARG(eig_top_supported(n, r) && batch >= 1, "eig_top: order must be in [1, 128] and 1 <= r <= min(16, n)");
   const size_t smem = eig_top_smem_bytes(n);
   const int    nt   = eig_threads(n);
-  auto         kern = nt == 128 ? eig_top_kernel<128> : (nt == 256 ? eig_top_kernel<256> : eig_top_kernel<512>);
+  auto         kern = nt == 128 ? eig_top_kernel<128, 1> : (nt == 512 ? eig_top_kernel<512, 1> : eig_top_kernel<256, 1>);
+  // more matrices than SMs: two CTAs per SM within 128 registers each take longer apiece and less in all.
+  // 600 matrices of 50, r = 4: 370 -> 246 us (284 with the shared-memory kernel before), 149 of them 149 ->
+  // 92; the others fit one CTA (n > 64) or several (n <= 32) as they are.
+  if (nt == 256 && batch > sm_count())
+    kern = eig_top_kernel<256, 2>;
   HF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<(unsigned)batch, nt, smem, s>>>(a, evecs, evals, info, n, r);
   note_launch();
