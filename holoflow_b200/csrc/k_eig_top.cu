@@ -28,6 +28,13 @@
 // needs are loaded ahead of it, and finished rows and columns are skipped.
 // Measured, 8 matrices, r = 4, before -> now: n = 32 86 -> 50 us, 64 172 -> 99, 128 396 -> 254 (at n = 64:
 // reduction 51 us, eigenvalues 14, factors and inverse iteration 20, back-transformation 6).
+// Accuracy: two solves per eigenvector (one with lambda to the rounding of ||T|| gains about 1e15; a third
+// changed no residual) and brackets that stop at 2^-54 ||T|| (the reduction has perturbed T by more).
+// Over Gram, decaying, cluttered and clustered spectra of n = 8 .. 128, r = 4, the residuals
+// ||A v - lambda v|| / ||A|| are 2.9e-16 .. 7.2e-16 in the median of a kind and at most 1.8e-15; the
+// shared-memory kernel before, with three solves, brackets relative to lambda and the library's square roots
+// and divisions, had 2.1e-16 .. 6.5e-16 and at most 2.0e-15.  The eigenvalues' errors agree (at most
+// 5.3e-15 ||A|| for both), and the filter matrix made from them is float32.
 // The eigenvalues ascend in evals[n - r .. n - 1] and the vectors go to the matching columns of
 // evecs ([n][n], column = eigenvalue index, as the Jacobi solver lays them out); the other entries
 // are not written.  info = 0, or 1 when the input is not finite.
