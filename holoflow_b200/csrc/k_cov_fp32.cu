@@ -16,7 +16,7 @@
 //    reduction: 331 -> 94 us.
 //  - float64: staged as x (exact in FP32) and widened as it is read; the block takes 128 registers, so
 //    one CTA per SM.  Measured, 16 windows of 50 x 16384 16-bit pixels: one thread per entry 2551 us, here
-//    110.
+//    94 with the reduction.
 #include <algorithm>
 
 #include "host/cov_split.hh"
@@ -183,16 +183,17 @@ __global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
   }
 }
 
-// Float64 reduction of the CTA partials in a fixed order (8 interleaved slices per entry, added
-// pairwise); undoes the shift exactly.  `blocked`: partials are the 8 x 8 upper blocks of
-// cov_cores_kernel, else whole [T][T] matrices of which the upper triangle is read.
-template <typename Acc>
+// Float64 reduction of the CTA partials in a fixed order (S interleaved slices per entry, added pairwise);
+// undoes the shift exactly.  `blocked`: partials are the 8 x 8 upper blocks of cov_cores_kernel, else whole
+// [T][T] matrices of which the upper triangle is read.
+template <typename Acc, int S>
 __global__ void __launch_bounds__(256) cov_reduce_kernel(const Acc *partial, const double *sums, int nblk, int nsum,
                                                          int T, int64_t P, double shift, int blocked, double *gram) {
-  __shared__ double red[3][8][32];
-  const int w = blockIdx.y, lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  constexpr int E = 256 / S; // entries per CTA
+  __shared__ double red[3][S][E];
+  const int w = blockIdx.y, lane = threadIdx.x % E, slice = threadIdx.x / E;
   const int NB = (T + 7) / 8, per = blocked ? NB * (NB + 1) / 2 * 64 : T * T;
-  const int e = blockIdx.x * 32 + lane;
+  const int e = blockIdx.x * E + lane;
   int       i = T, j = T;
   if (e < per) {
     if (blocked) {
@@ -210,11 +211,11 @@ __global__ void __launch_bounds__(256) cov_reduce_kernel(const Acc *partial, con
   double     s = 0.0, si = 0.0, sj = 0.0;
   if (ok) {
     const Acc *pp = partial + (int64_t)w * nblk * per + e;
-    for (int b = slice; b < nblk; b += 8)
+    for (int b = slice; b < nblk; b += S)
       s += (double)pp[(int64_t)b * per];
     if (shift != 0.0) {
       const double *sp = sums + (int64_t)w * nsum * T;
-      for (int b = slice; b < nsum; b += 8)
+      for (int b = slice; b < nsum; b += S)
         si += sp[(int64_t)b * T + i], sj += sp[(int64_t)b * T + j];
     }
   }
@@ -224,9 +225,13 @@ __global__ void __launch_bounds__(256) cov_reduce_kernel(const Acc *partial, con
     return;
   double t[3];
 #pragma unroll
-  for (int q = 0; q < 3; ++q)
-    t[q] = ((red[q][0][lane] + red[q][1][lane]) + (red[q][2][lane] + red[q][3][lane])) +
-           ((red[q][4][lane] + red[q][5][lane]) + (red[q][6][lane] + red[q][7][lane]));
+  for (int q = 0; q < 3; ++q) {
+    if constexpr (S == 8)
+      t[q] = ((red[q][0][lane] + red[q][1][lane]) + (red[q][2][lane] + red[q][3][lane])) +
+             ((red[q][4][lane] + red[q][5][lane]) + (red[q][6][lane] + red[q][7][lane]));
+    else
+      t[q] = red[q][0][lane];
+  }
   // x_i x_j = c_i c_j + s (c_i + c_j) + s^2 with c = x - s; the sums are of c (blocked) or of x
   const double sq = shift * shift * (double)P;
   const double v  = shift != 0.0 ? t[0] + (shift * (t[1] + t[2]) + (blocked ? sq : -sq)) : t[0];
@@ -238,7 +243,13 @@ template <typename Acc>
 int launch_reduce(const Acc *partial, const double *sums, int nblk, int nsum, int T, int64_t P, double shift, int blocked,
                   double *gram, int nwin, cudaStream_t s) {
   const int NB = (T + 7) / 8, per = blocked ? NB * (NB + 1) / 2 * 64 : T * T;
-  cov_reduce_kernel<<<dim3((per + 31) / 32, nwin), 256, 0, s>>>(partial, sums, nblk, nsum, T, P, shift, blocked, gram);
+  // 8 slices keep the loads of a window's hundreds of partials in flight; where few partials meet more
+  // CTAs than run at once, a thread per entry takes them all: 64 windows of T = 128 with 5 partials 48 -> 9.4
+  // us, 16 with 18 18 -> 7.2; below that line 16 windows of T = 64 with 18 take 5.9 sliced, 6.8 not
+  const bool sliced = nblk >= 32 || (int64_t)((per + 31) / 32) * nwin <= 8LL * sm_count();
+  auto       kern   = sliced ? cov_reduce_kernel<Acc, 8> : cov_reduce_kernel<Acc, 1>;
+  const int  E      = sliced ? 32 : 256;
+  kern<<<dim3((per + E - 1) / E, nwin), 256, 0, s>>>(partial, sums, nblk, nsum, T, P, shift, blocked, gram);
   note_launch();
   return launch_status("cov_reduce_kernel");
 }

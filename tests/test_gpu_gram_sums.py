@@ -86,3 +86,17 @@ def test_noalloc_calls_without_workspace_overlap(cuda, rng):
     torch.cuda.synchronize()
     for s, x, dev, dt, g in jobs:
         _check(g.cpu().numpy(), x, "u16")
+
+
+# Many windows with few partials, few with many, and the batches on either side of a full wave of CTAs.
+# Samples within 8 of the shift: every FP32 sum is a small integer, so the matrix is exact however it is
+# split and reduced.
+@pytest.mark.parametrize("fmt,B,T,P", [("u16", 64, 128, 1024), ("u16", 16, 64, 16384), ("u8", 7, 128, 1024), ("u16", 9, 32, 8192),
+                                       ("f32", 296, 32, 512), ("u16", 297, 32, 64), ("mono12p", 1, 128, 65536)])
+def test_split_and_reduction_of_fp32_sums(cuda, rng, fmt, B, T, P):
+    from holoflow_b200 import pipeline as pl
+    x = rng.integers(-8, 9, (B, T, P)).astype(np.float64) + {"u8": 128, "u16": 2048, "mono12p": 2048, "f32": 0}[fmt]
+    dev, dt = _device(x, fmt)
+    got = pl.covariance(dev, dt, B, T, P).cpu().numpy()
+    for b in range(B):
+        assert np.array_equal(got[b], x[b] @ x[b].T)
