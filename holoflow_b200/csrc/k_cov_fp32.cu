@@ -30,6 +30,7 @@ constexpr int kCovThr = 256;
 
 struct CovGeom {
   int NB, U, G, PX, XS; // 8-frame blocks, upper blocks, pixel groups, pixels per tile, row stride
+  int lh;               // 2^lh lanes add the groups' sums of an entry
   int nxs;              // floats of the tile (and of the final block rows, 8 sums per thread)
   size_t smem;
 };
@@ -44,6 +45,8 @@ CovGeom cov_geom(int T) {
     if ((size_t)px * g.XS * sizeof(float) <= 48 * 1024 && waste < best - 1e-9)
       best = waste, g.PX = px;
   }
+  for (g.lh = 0; g.lh < 5 && (2 << g.lh) * g.U * 8 <= kCovThr;)
+    ++g.lh;
   g.nxs  = std::max(g.PX * g.XS, 2 * 8 * kCovThr);
   g.smem = (size_t)g.nxs * sizeof(float) + 128 * (sizeof(int64_t) + sizeof(unsigned long long));
   return g;
@@ -165,11 +168,26 @@ __global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
       for (int j = 0; j < 8; ++j)
         rows[tid * 8 + j] = acc[i][j];
     __syncthreads();
-    for (int e = tid; e < g.U * 8; e += kCovThr) {
-      double s = 0.0;
-      for (int q = 0; q < g.G; ++q)
-        s += (double)rows[q * g.U * 8 + e];
-      partial[pidx + (e >> 3) * 64 + 8 * i + (e & 7)] = (Acc)s;
+    if constexpr (sizeof(Acc) == 4) {
+      for (int e = tid; e < g.U * 8; e += kCovThr) {
+        double s = 0.0;
+        for (int q = 0; q < g.G; ++q)
+          s += (double)rows[q * g.U * 8 + e];
+        partial[pidx + (e >> 3) * 64 + 8 * i + (e & 7)] = (Acc)s;
+      }
+    } else { // few blocks have many groups (256 at T <= 8: 64 windows of 1024 pixels 44 us in all, 27 by lanes)
+      for (int k0 = 0; k0 < (g.U * 8) << g.lh; k0 += kCovThr) { // whole warps take part in the shuffles
+        const int  k = k0 + tid, e = k >> g.lh, h = k & ((1 << g.lh) - 1);
+        const bool in = e < g.U * 8;
+        Acc        s = Acc(0);
+        if (in)
+          for (int q = h; q < g.G; q += 1 << g.lh)
+            s += rows[q * g.U * 8 + e];
+        for (int o = (1 << g.lh) >> 1; o > 0; o >>= 1)
+          s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (in && h == 0)
+          partial[pidx + (e >> 3) * 64 + 8 * i + (e & 7)] = s;
+      }
     }
     __syncthreads();
   }

@@ -96,7 +96,7 @@ int hf_temporal_dft(const void *in, int in_dtype, int64_t batch, int T, int64_t 
  * (of x - shift, undone exactly; one FP32 partial per CTA), every other input in float64 (exact for
  * integer samples up to 2^53).
  * `ws` must hold hf_covariance_workspace_bytes(T, P) bytes per batch item.  It may be NULL for the
- * inputs summed in float64: these then take the direct kernel (one thread per entry, no workspace), as
+ * inputs summed in float64: these then take the direct kernel (no workspace), as
  * T > 128 does always. */
 size_t hf_covariance_workspace_bytes(int T, int64_t P);
 int    hf_covariance(const void *in, int in_dtype, int64_t batch, int T, int64_t P, double *gram,

@@ -43,7 +43,8 @@ def _check(got, x, fmt):
     ("u16", 1, 1, 5, 0), ("u16", 2, 3, 1000, 0), ("u8", 2, 16, 333, 0), ("mono12p", 2, 17, 4098, 0),
     ("u16", 300, 50, 700, 0), ("u16", 1, 50, 300001, 0), ("f32", 2, 50, 20000, 0), ("f32", 300, 9, 257, 0),
     ("u8", 2, 100, 5000, 0), ("f32", 1, 127, 3001, 0), ("mono12p", 1, 127, 3002, 0), ("u16", 2, 32, 4099, 0),
-    ("u16", 2, 64, 4096, 2), ("u8", 2, 64, 4096, 3), ("mono12p", 2, 128, 2048, 1), ("f32", 2, 128, 1001, 0)])
+    ("u16", 2, 64, 4096, 2), ("u8", 2, 64, 4096, 3), ("mono12p", 2, 128, 2048, 1), ("f32", 2, 128, 1001, 0),
+    ("u16", 2, 130, 600, 0), ("f32", 1, 200, 777, 0), ("u8", 64, 8, 1024, 0), ("mono12p", 3, 24, 254, 0)])
 def test_float64_sums(cuda, rng, fmt, B, T, P, lead):
     from holoflow_b200 import pipeline as pl
     import torch
