@@ -75,7 +75,7 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_
                : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T over signed int8 operands with an int32 accumulator.
+// D[tmem] (+)= A[smem] * B[smem]^T over unsigned 8-bit operands with a 32-bit accumulator that wraps.
 __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                        uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
