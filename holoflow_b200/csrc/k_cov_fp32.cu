@@ -14,9 +14,10 @@
 //    the kernel).  Two CTAs of 256 threads per SM (the registers of 288 threads fit once, whose load
 //    latency nothing covers: 165 us).  Measured, 2 windows of 32 x 600 x 800 16-bit frames, kernel +
 //    reduction: 331 -> 94 us.
-//  - float64: staged as x (exact in FP32) and widened as it is read; the block takes 128 registers, so
-//    one CTA per SM.  Measured, 16 windows of 50 x 16384 16-bit pixels: one thread per entry 2551 us, here
-//    94 with the reduction.
+//  - float64: staged as x and widened as it is read; the block takes 128 registers, so one CTA per SM, and
+//    three times the loads in flight cover for the second (12-bit frames spill with them).  Measured, 2 windows
+//    of 50 x 600 x 800 16-bit frames: 275 us (in FP32 180; float64 needs 96 at its pipe's rate), 16 of 50 x 16384
+//    91 with the reduction, 2551 with a thread per entry.
 #include <algorithm>
 
 #include "host/cov_split.hh"
@@ -66,11 +67,21 @@ template <int FMT> __device__ __forceinline__ uint32_t raw_sample(const uint8_t 
   }
 }
 
+// A staged sample as an operand.  For float64 sums integers stay integers in the tile and become 2^52 + v by
+// their bits, 2^52 taken off: one instruction of the FP64 pipe instead of a conversion (308 -> 288 us for those 2 windows).
+template <int FMT, typename Acc> __device__ __forceinline__ Acc widen(float x) {
+  if constexpr (FMT != HF_F32 && sizeof(Acc) == 8)
+    return __hiloint2double(0x43300000, __float_as_int(x)) - 4503599627370496.0;
+  else
+    return (Acc)x;
+}
+
 // Acc: float, or double with shift = 0 and no frame sums.
 template <int FMT, typename Acc>
 __global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
     cov_cores_kernel(FrameRing ring, int T, int64_t P, float shift, CovGeom g, Acc *partial, double *sums) {
   constexpr bool kShift = FMT != HF_F32 && sizeof(Acc) == 4;
+  constexpr bool kRaw   = !kShift; // the tile holds the samples' bits
   extern __shared__ __align__(16) float xs[]; // [PX][XS]
   int64_t            *foff = reinterpret_cast<int64_t *>(xs + g.nxs);                // [128]
   unsigned long long *ssum = reinterpret_cast<unsigned long long *>(foff + 128);     // [128]
@@ -99,11 +110,13 @@ __global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
   const int     items  = 2 * g.NB * g.PX; // (frame quad, pixel), pixel fastest
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t p0 = tile * g.PX;
-    constexpr int V = 4; // frame quads in flight per thread
+    constexpr int V = sizeof(Acc) == 4 || FMT == HF_MONO12P ? 4 : 12; // frame quads in flight per thread
     for (int i0 = tid & ~31; i0 < items; i0 += V * kCovThr) { // whole warps: PX is a multiple of 32
       uint32_t v[V][4];
 #pragma unroll
       for (int u = 0; u < V; ++u) { // unconditional loads (clamped addresses), so that all are in flight
+        if (V > 4 && i0 + u * kCovThr >= items)
+          break; // (a whole warp's; of 4 at most 3 repeat the last items)
         const int     it = min(i0 + u * kCovThr, items - 32), tq = it / g.PX, p = it - tq * g.PX + (tid & 31);
         const int64_t pc = min(p0 + p, P - 1);
 #pragma unroll
@@ -117,8 +130,8 @@ __global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
           float x[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const float c = FMT == HF_F32 ? __uint_as_float(v[u][q])
-                                          : __uint_as_float(0x4B000000u | v[u][q]) - (8388608.f + shift);
+            const float c = kRaw ? __uint_as_float(v[u][q])
+                                 : __uint_as_float(0x4B000000u | v[u][q]) - (8388608.f + shift);
             x[q]          = p0 + p < P && 4 * tq + q < T ? c : 0.f;
           }
           *reinterpret_cast<float4 *>(xs + p * g.XS + 4 * tq) = make_float4(x[0], x[1], x[2], x[3]);
@@ -146,8 +159,10 @@ __global__ void __launch_bounds__(kCovThr, sizeof(Acc) == 4 ? 2 : 1)
       for (int p = grp; p < g.PX; p += g.G) {
         const float4 a0 = *reinterpret_cast<const float4 *>(xa + p * g.XS), a1 = *reinterpret_cast<const float4 *>(xa + p * g.XS + 4);
         const float4 b0 = *reinterpret_cast<const float4 *>(xb + p * g.XS), b1 = *reinterpret_cast<const float4 *>(xb + p * g.XS + 4);
-        const Acc    va[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const Acc    vb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        const Acc    va[8] = {widen<FMT, Acc>(a0.x), widen<FMT, Acc>(a0.y), widen<FMT, Acc>(a0.z), widen<FMT, Acc>(a0.w),
+                              widen<FMT, Acc>(a1.x), widen<FMT, Acc>(a1.y), widen<FMT, Acc>(a1.z), widen<FMT, Acc>(a1.w)};
+        const Acc    vb[8] = {widen<FMT, Acc>(b0.x), widen<FMT, Acc>(b0.y), widen<FMT, Acc>(b0.z), widen<FMT, Acc>(b0.w),
+                              widen<FMT, Acc>(b1.x), widen<FMT, Acc>(b1.y), widen<FMT, Acc>(b1.z), widen<FMT, Acc>(b1.w)};
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
